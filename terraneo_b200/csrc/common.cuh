@@ -95,6 +95,14 @@ int mesh_create_diamonds( const ShellTopology& t, double r_min, double r_max, in
 
 }  // namespace tn
 
+// Lateral stencils and radial factors of an operator whose wedge matrices
+// separate (lateral.cuh), in double and single precision, built on first use.
+struct tn_lateral_tables
+{
+    double *lat = nullptr, *rad = nullptr;
+    float * lat32 = nullptr, *rad32 = nullptr;
+};
+
 // The mesh object behind the opaque tn_mesh handle.
 struct tn_mesh
 {
@@ -117,6 +125,7 @@ struct tn_mesh
     // duplicated lateral positions, CSR: members of group g are
     // halo_members[halo_offsets[g] .. halo_offsets[g+1]) as lateral indices
     int  n_halo_groups    = 0;
+    int  n_halo_members   = 0;
     int* d_halo_offsets   = nullptr;
     int* d_halo_members   = nullptr;
     int* d_lat_group      = nullptr; // halo group of each lateral position, -1 if not duplicated
@@ -129,8 +138,10 @@ struct tn_mesh
     // flipped (the orientation test against the neighbour's centre), built on first use
     uint8_t* d_fv_orient = nullptr;
 
-    // lateral quadrature tables of the gradient-form operators (Laplace,
-    // DivKGrad, VectorLaplace), built on first use: [10][N][N][2 wedges][105]
+    tn_lateral_tables laplace_tables, mass_tables;
+
+    // lateral quadrature table of DivKGrad, built on first use:
+    // [10][N][N][2 wedges][84]
     std::mutex      geom_mutex;
     double*         d_grad_geom = nullptr;
     double*         d_stokes_geom = nullptr; // Divergence / Gradient, this mesh as the velocity mesh

@@ -10,12 +10,10 @@
 #include <cmath>
 
 #include "common.cuh"
+#include "lateral.cuh"
 #include "wedge.cuh"
 
 namespace tn {
-
-template < typename T >
-int halo_sum( const tn_mesh* m, T* const* fields, int nfields, cudaStream_t st );
 
 namespace {
 
@@ -28,34 +26,18 @@ constexpr double kQP32Host[3][2] = { { 0.6666666666666666, 0.1666666666666667 },
 constexpr double kZeta32 = 0.5773502691896257;
 constexpr double kW32    = 0.1666666666666667;
 
-// Coupling of a cell's wedge nodes: all (kNeu), CMB-side nodes decoupled
-// keeping their diagonal (kBot), SURFACE-side ones likewise (kTop), or the
-// diagonal alone (kDiag).  It depends on the cell's radial layer only.
-enum : int
-{
-    kNeu  = 0,
-    kBot  = 1,
-    kTop  = 2,
-    kDiag = 3
-};
-
 template < typename T >
 struct GradParams
 {
     int             N, n1;
     const double*   geom; // lateral quadrature table, kGeomStride doubles per wedge
     const T*        radii;
-    const T*        k; // nodal coefficient (DivKGrad) or NULL
-    Ptr3< const T > src;
-    Ptr3< T >       dst;
+    const T*        k; // nodal coefficient
+    const T*        src;
+    T*              dst;
     int             mode_first, mode_inner, mode_last; // coupling of layer 0, 1..N-2, N-1
     int             single;                            // 1-point rule instead of 3x2
 };
-
-__device__ __forceinline__ int layer_mode( int r, int N, int first, int inner, int last )
-{
-    return r == 0 ? first : ( r == N - 1 ? last : inner );
-}
 
 // Factored wedge stiffness.  For x = r(zeta) ((1-xi-eta) p0 + xi p1 + eta p2)
 // with a = p1 - p0, b = p2 - p0, v = a x b, c = p0 + xi a + eta b and
@@ -68,15 +50,17 @@ __device__ __forceinline__ int layer_mode( int r, int N, int first, int inner, i
 // A quadrature point's contribution w |det J| g_i . g_j therefore splits into
 // lateral factors (u_m . u_m', lat_m lat_m' |v|^2, (u_m . v) lat_m', all
 // / |D|) times radial ones (h nr_i nr_j, r^2 / h, r nr), and on the
-// tensor-product 3x2 rule the lateral and radial sums separate.  The lateral
-// factors depend only on the triangle, so they are tabulated once per mesh:
-// set 0 is the sum over the three lateral points of the 3x2 rule with weight
-// 1/6, sets 1-3 the points one by one and set 4 the centroid (weights
-// applied in the kernel).  Each set is U (6, symmetric), Lam (6, symmetric),
-// W (9, row-major).  Mathematically the same stiffness as the per-point
-// Jacobian of fe/wedge/integrands.hpp, evaluated with far fewer operations.
+// tensor-product 3x2 rule the lateral and radial sums separate: with a
+// constant coefficient (Laplace, VectorLaplace) the whole operator is a sum of
+// lateral stencils times radial factors (LaplaceOp, lateral.cuh).  DivKGrad's
+// nodal k keeps the points apart: the lateral factors depend only on the
+// triangle, so they are tabulated once per mesh, sets 0-2 for the three
+// lateral points of the 3x2 rule and set 3 for the centroid (weights applied
+// in the kernel).  Each set is U (6, symmetric), Lam (6, symmetric), W (9,
+// row-major).  Mathematically the same stiffness as the per-point Jacobian of
+// fe/wedge/integrands.hpp, evaluated with far fewer operations.
 constexpr int kGeomSet    = 21;
-constexpr int kGeomStride = 5 * kGeomSet;
+constexpr int kGeomStride = 4 * kGeomSet;
 
 // radial factors of one set: R[li + lj] (bottom/top node pairs), S2, P[l]
 template < typename T >
@@ -116,11 +100,10 @@ __host__ __device__ constexpr int sym6( int i, int j )
 
 // One thread per cell (r fastest: neighbouring threads share the lateral
 // table entry and touch consecutive addresses).  Each wedge's symmetric 6x6
-// matrix is formed from its table entry and the layer's radial factors and
-// applied to all NC components; the 8 node sums of the cell are kept in
-// registers and added with one atomic per node and component.
-template < typename T, int NC, bool HAS_K >
-__global__ void __launch_bounds__( 128 ) grad_cell_kernel( GradParams< T > P )
+// matrix is formed from its table entry and the layer's radial factors; the 8
+// node sums of the cell are kept in registers and added with one atomic each.
+template < typename T >
+__global__ void __launch_bounds__( 128 ) divkgrad_cell_kernel( GradParams< T > P )
 {
     const int       N = P.N, n1 = P.n1;
     const long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x;
@@ -139,25 +122,21 @@ __global__ void __launch_bounds__( 128 ) grad_cell_kernel( GradParams< T > P )
     for ( int n = 0; n < 6; ++n )
         cpl[n] = mode == kNeu || ( mode == kBot && n >= 3 ) || ( mode == kTop && n < 3 );
 
-    T out[NC][2][2][2];
-#pragma unroll
-    for ( int c = 0; c < NC; ++c )
-        for ( int i = 0; i < 8; ++i )
-            ( &out[c][0][0][0] )[i] = T( 0 );
+    T out[2][2][2];
+    for ( int i = 0; i < 8; ++i )
+        ( &out[0][0][0] )[i] = T( 0 );
 #pragma unroll
     for ( int w = 0; w < 2; ++w )
     {
         const double* G = P.geom + ( ( ( size_t( d ) * N + x ) * N + y ) * 2 + w ) * kGeomStride;
-        T             s[NC][6], kv[6];
+        T             s[6], kv[6];
 #pragma unroll
         for ( int n = 0; n < 6; ++n )
         {
             const size_t i = lat_index( n1, d, x + kWedgeNode[w][n][0], y + kWedgeNode[w][n][1] ) * n1 + r +
                              kWedgeNode[w][n][2];
-#pragma unroll
-            for ( int c = 0; c < NC; ++c )
-                s[c][n] = P.src.p[c][i];
-            kv[n] = HAS_K ? P.k[i] : T( 1 );
+            s[n]  = P.src[i];
+            kv[n] = P.k[i];
         }
         T A[21];
 #pragma unroll
@@ -166,30 +145,13 @@ __global__ void __launch_bounds__( 128 ) grad_cell_kernel( GradParams< T > P )
         if ( P.single )
         {
             // quad_felippa_1x1: (1/3, 1/3, 0), weight 1; k at the centroid is the mean of the six
-            T ke = T( 1 );
-            if ( HAS_K )
-                ke = ( kv[0] + kv[1] + kv[2] + kv[3] + kv[4] + kv[5] ) * T( 1.0 / 6.0 );
+            const T    ke = ( kv[0] + kv[1] + kv[2] + kv[3] + kv[4] + kv[5] ) * T( 1.0 / 6.0 );
             const T    rm = r1 + h;
             Radial< T > f;
             f.R[0] = f.R[1] = f.R[2] = ke * h * T( 0.25 );
             f.S2                     = ke * rm * rm / h;
             f.P[0] = f.P[1] = ke * rm * T( 0.5 );
-            add_set( A, G + 4 * kGeomSet, f );
-        }
-        else if ( !HAS_K )
-        {
-            Radial< T > f{};
-#pragma unroll
-            for ( int zq = 0; zq < 2; ++zq )
-            {
-                const T zeta = zq ? T( kZeta32 ) : T( -kZeta32 );
-                const T nb = T( 0.5 ) * ( T( 1 ) - zeta ), nt = T( 0.5 ) * ( T( 1 ) + zeta );
-                const T rr = r1 + h * ( T( 1 ) + zeta );
-                f.R[0] += h * nb * nb, f.R[1] += h * nb * nt, f.R[2] += h * nt * nt;
-                f.S2 += rr * rr / h;
-                f.P[0] += rr * nb, f.P[1] += rr * nt;
-            }
-            add_set( A, G, f );
+            add_set( A, G + 3 * kGeomSet, f );
         }
         else
         {
@@ -211,38 +173,132 @@ __global__ void __launch_bounds__( 128 ) grad_cell_kernel( GradParams< T > P )
                     f.S2 += wk * rr * rr / h;
                     f.P[0] += wk * rr * nb, f.P[1] += wk * rr * nt;
                 }
-                add_set( A, G + ( 1 + q ) * kGeomSet, f );
+                add_set( A, G + q * kGeomSet, f );
             }
         }
+        T sc[6];
 #pragma unroll
-        for ( int c = 0; c < NC; ++c )
+        for ( int n = 0; n < 6; ++n )
+            sc[n] = cpl[n] ? s[n] : T( 0 );
+#pragma unroll
+        for ( int i = 0; i < 6; ++i )
         {
-            T sc[6];
+            T acc = T( 0 );
 #pragma unroll
-            for ( int n = 0; n < 6; ++n )
-                sc[n] = cpl[n] ? s[c][n] : T( 0 );
-#pragma unroll
-            for ( int i = 0; i < 6; ++i )
-            {
-                T acc = T( 0 );
-#pragma unroll
-                for ( int j = 0; j < 6; ++j )
-                    acc += A[sym6( i, j )] * sc[j];
-                if ( !cpl[i] )
-                    acc = A[sym6( i, i )] * s[c][i];
-                out[c][kWedgeNode[w][i][0]][kWedgeNode[w][i][1]][kWedgeNode[w][i][2]] += acc;
-            }
+            for ( int j = 0; j < 6; ++j )
+                acc += A[sym6( i, j )] * sc[j];
+            if ( !cpl[i] )
+                acc = A[sym6( i, i )] * s[i];
+            out[kWedgeNode[w][i][0]][kWedgeNode[w][i][1]][kWedgeNode[w][i][2]] += acc;
         }
     }
-#pragma unroll
-    for ( int c = 0; c < NC; ++c )
-        for ( int dx = 0; dx < 2; ++dx )
-            for ( int dy = 0; dy < 2; ++dy )
-                for ( int dz = 0; dz < 2; ++dz )
-                    atomicAdd( P.dst.p[c] + lat_index( n1, d, x + dx, y + dy ) * n1 + r + dz, out[c][dx][dy][dz] );
+    for ( int dx = 0; dx < 2; ++dx )
+        for ( int dy = 0; dy < 2; ++dy )
+            for ( int dz = 0; dz < 2; ++dz )
+                atomicAdd( P.dst + lat_index( n1, d, x + dx, y + dy ) * n1 + r + dz, out[dx][dy][dz] );
 }
 
-// Host tabulation of the lateral factors (double), one entry per wedge.
+// The lateral factors of a triangle at a lateral point with sig = 1 / |D|: u[3] and lat[3] (factored stiffness
+// above); v = a x b.
+struct LateralTriangle
+{
+    double a[3], b[3], v[3], p0[3], sig;
+    __host__ __device__ LateralTriangle( const double* q0, const double* q1, const double* q2 )
+    {
+        for ( int k = 0; k < 3; ++k )
+            p0[k] = q0[k], a[k] = q1[k] - q0[k], b[k] = q2[k] - q0[k];
+        cross( a, b, v );
+        sig = 1.0 / fabs( dot( v, p0 ) );
+    }
+    __host__ __device__ void at( double xi, double eta, double u[3][3], double lat[3] ) const
+    {
+        double c[3];
+        for ( int k = 0; k < 3; ++k )
+            c[k] = p0[k] + xi * a[k] + eta * b[k];
+        cross( b, c, u[1] );
+        cross( c, a, u[2] );
+        for ( int k = 0; k < 3; ++k )
+            u[0][k] = -( u[1][k] + u[2][k] );
+        lat[0] = 1.0 - xi - eta, lat[1] = xi, lat[2] = eta;
+    }
+    static __host__ __device__ void cross( const double* x, const double* y, double* o )
+    {
+        o[0] = x[1] * y[2] - x[2] * y[1];
+        o[1] = x[2] * y[0] - x[0] * y[2];
+        o[2] = x[0] * y[1] - x[1] * y[0];
+    }
+    static __host__ __device__ double dot( const double* x, const double* y ) { return x[0] * y[0] + x[1] * y[1] + x[2] * y[2]; }
+};
+
+// A layer's two rows of the Laplacian from the lateral sums of its levels with
+// the stencils U, W^T (per level; rows sum to zero because sum_m u_m = 0) and
+// Lam, W (on the difference of the levels), all summed over the 3x2 rule's
+// lateral points with weight 1/6, and its radial factors R[0] = R[2], R[1],
+// S2 / 4, P[0] / 2, P[1] / 2: add_set's entries, both rows sharing the differences.
+// Apply with its halo, FP64, before (one thread per cell, atomics) and now:
+// Laplace 112 -> 39 us at level 6, 911 -> 271 us at level 7 (1.3 TB/s of its
+// 16 bytes per node); VectorLaplace 228 -> 118 us at level 6; FP32 Laplace
+// 84 -> 25 us at level 6.
+template < typename T >
+struct LaplaceOp
+{
+    static constexpr int           S = 2, D = 2, K = S + D, R = 5;
+    static constexpr bool          kDiff = true;
+    static __device__ __forceinline__ void layer( const T ( &f )[R], const T ( &b )[S], const T ( &t )[S], const T ( &d )[D + 1],
+                                                  T& low, T& high )
+    {
+        const T x = f[2] * d[0], e = f[3] * b[1] + f[4] * t[1];
+        low  = f[0] * b[0] + f[1] * t[0] - x + f[3] * d[1] - e;
+        high = f[0] * t[0] + f[1] * b[0] + x + f[4] * d[1] + e;
+    }
+    static __device__ __forceinline__ T side_low( const T ( &f )[R], const T ( &s )[S], const T ( &v )[D + 1] )
+    {
+        return f[0] * s[0] + f[2] * v[0] - f[3] * ( v[1] + s[1] );
+    }
+    static __device__ __forceinline__ T side_high( const T ( &f )[R], const T ( &s )[S], const T ( &v )[D + 1] )
+    {
+        return f[0] * s[0] + f[2] * v[0] + f[4] * ( v[1] + s[1] );
+    }
+    static __device__ __forceinline__ T self_low( const T ( &f )[R], const T ( &v )[K] )
+    {
+        return f[0] * v[0] + f[2] * v[2] - f[3] * ( v[3] + v[1] );
+    }
+    static __device__ __forceinline__ T self_high( const T ( &f )[R], const T ( &v )[K] )
+    {
+        return f[0] * v[0] + f[2] * v[2] + f[4] * ( v[3] + v[1] );
+    }
+    // adds the factors between vertices i and j of a triangle
+    static __device__ void triangle( const double* p0, const double* p1, const double* p2, int i, int j, double* A )
+    {
+        const LateralTriangle tri( p0, p1, p2 );
+        const double   vv = LateralTriangle::dot( tri.v, tri.v );
+        for ( int q = 0; q < 3; ++q )
+        {
+            double u[3][3], l[3];
+            tri.at( kQP32[q][0], kQP32[q][1], u, l );
+            const double f = kW32 * tri.sig;
+            A[0] += f * LateralTriangle::dot( u[i], u[j] );
+            A[1] += f * LateralTriangle::dot( u[j], tri.v ) * l[i];
+            A[2] += f * l[i] * l[j] * vv;
+            A[3] += f * LateralTriangle::dot( u[i], tri.v ) * l[j];
+        }
+    }
+    static __device__ void radial( double r1, double r2, double* f )
+    {
+        const double h = 0.5 * ( r2 - r1 );
+        for ( int k = 0; k < R; ++k )
+            f[k] = 0.0;
+        for ( int zq = 0; zq < 2; ++zq )
+        {
+            const double zeta = zq ? kZeta32 : -kZeta32, nb = 0.5 * ( 1.0 - zeta ), nt = 0.5 * ( 1.0 + zeta );
+            const double rr   = r1 + h * ( 1.0 + zeta );
+            f[0] += h * nb * nb, f[1] += h * nb * nt, f[2] += 0.25 * rr * rr / h;
+            f[3] += 0.5 * rr * nb, f[4] += 0.5 * rr * nt;
+        }
+    }
+};
+
+// Host tabulation of DivKGrad's lateral factors (double), one entry per wedge.
 void build_grad_geometry( const tn_mesh* m, std::vector< double >& G )
 {
     const int    N = m->N, n1 = m->n1;
@@ -251,12 +307,6 @@ void build_grad_geometry( const tn_mesh* m, std::vector< double >& G )
                                  { kQP32Host[1][0], kQP32Host[1][1] },
                                  { kQP32Host[2][0], kQP32Host[2][1] },
                                  { 1.0 / 3.0, 1.0 / 3.0 } };
-    auto cross = []( const double* a, const double* b, double* o ) {
-        o[0] = a[1] * b[2] - a[2] * b[1];
-        o[1] = a[2] * b[0] - a[0] * b[2];
-        o[2] = a[0] * b[1] - a[1] * b[0];
-    };
-    auto dotp = []( const double* a, const double* b ) { return a[0] * b[0] + a[1] * b[1] + a[2] * b[2]; };
     G.assign( size_t( kDiamonds ) * N * N * 2 * kGeomStride, 0.0 );
     for ( int d = 0; d < kDiamonds; ++d )
         for ( int x = 0; x < N; ++x )
@@ -267,39 +317,22 @@ void build_grad_geometry( const tn_mesh* m, std::vector< double >& G )
                     const double* p[3];
                     for ( int k = 0; k < 3; ++k )
                         p[k] = m->h_coords.data() + lat_index( n1, d, x + wn[w][k][0], y + wn[w][k][1] ) * 3;
-                    double a[3], b[3], v[3];
-                    for ( int k = 0; k < 3; ++k )
-                        a[k] = p[1][k] - p[0][k], b[k] = p[2][k] - p[0][k];
-                    cross( a, b, v );
-                    const double sig = 1.0 / std::fabs( dotp( v, p[0] ) ), vv = dotp( v, v );
+                    const LateralTriangle tri( p[0], p[1], p[2] );
+                    const double   vv = LateralTriangle::dot( tri.v, tri.v );
                     for ( int q = 0; q < 4; ++q )
                     {
-                        const double xi = pts[q][0], eta = pts[q][1];
-                        const double lat[3] = { 1.0 - xi - eta, xi, eta };
-                        double       c[3], u[3][3];
-                        for ( int k = 0; k < 3; ++k )
-                            c[k] = p[0][k] + xi * a[k] + eta * b[k];
-                        cross( b, c, u[1] );
-                        cross( c, a, u[2] );
-                        for ( int k = 0; k < 3; ++k )
-                            u[0][k] = -( u[1][k] + u[2][k] );
-                        double set[kGeomSet];
-                        int    e = 0;
+                        double u[3][3], lat[3];
+                        tri.at( pts[q][0], pts[q][1], u, lat );
+                        double* set = g + q * kGeomSet;
                         for ( int i = 0; i < 3; ++i )
                             for ( int j = i; j < 3; ++j )
-                                set[e++] = sig * dotp( u[i], u[j] );
+                                *set++ = tri.sig * LateralTriangle::dot( u[i], u[j] );
                         for ( int i = 0; i < 3; ++i )
                             for ( int j = i; j < 3; ++j )
-                                set[e++] = sig * lat[i] * lat[j] * vv;
+                                *set++ = tri.sig * lat[i] * lat[j] * vv;
                         for ( int i = 0; i < 3; ++i )
                             for ( int j = 0; j < 3; ++j )
-                                set[e++] = sig * dotp( u[i], v ) * lat[j];
-                        for ( int k = 0; k < kGeomSet; ++k )
-                        {
-                            g[( 1 + q ) * kGeomSet + k] = set[k];
-                            if ( q < 3 )
-                                g[k] += kW32 * set[k];
-                        }
+                                *set++ = tri.sig * LateralTriangle::dot( u[i], tri.v ) * lat[j];
                     }
                 }
 }
@@ -327,47 +360,27 @@ const double* grad_geometry( const tn_mesh* m )
 
 }  // namespace
 
-// Shared driver: Replace zeroes dst, the cell kernel accumulates, and the
-// additive communication mode sums duplicated nodes.
-template < typename T, int NC >
-int grad_family_apply( const tn_mesh* m, const T* k, const T* const* src, T* const* dst, int mode_first,
-                       int mode_inner, int mode_last, int single, int apply_mode, int comm_mode, cudaStream_t st,
-                       const char* what )
+// Laplace / VectorLaplace driver (lateral.cuh).
+template < typename T >
+int constant_gradient_apply( const tn_mesh* m, int nc, const T* const* src, T* const* dst, int mode_first, int mode_inner,
+                             int mode_last, int apply_mode, int comm_mode, cudaStream_t st, const char* what )
 {
     TN_CHECK_ARG( m && src && dst, std::string( what ) + ": null argument" );
     TN_CHECK_ARG( apply_mode == TN_APPLY_REPLACE || apply_mode == TN_APPLY_ADD, std::string( what ) + ": bad apply mode" );
-    GradParams< T > P{};
-    for ( int c = 0; c < 3; ++c )
-    {
-        P.src.p[c] = nullptr;
-        P.dst.p[c] = nullptr;
-    }
-    for ( int c = 0; c < NC; ++c )
+    LateralParams< T > P{};
+    for ( int c = 0; c < nc; ++c )
     {
         TN_CHECK_ARG( src[c] && dst[c], std::string( what ) + ": null field pointer" );
         P.src.p[c] = src[c];
         P.dst.p[c] = dst[c];
-        if ( apply_mode == TN_APPLY_REPLACE )
-            TN_CUDA_TRY( cudaMemsetAsync( dst[c], 0, m->ns * sizeof( T ), st ) );
     }
-    P.N = m->N, P.n1 = m->n1, P.geom = grad_geometry( m );
-    if ( !P.geom )
+    if ( !lateral_tables< LaplaceOp< T > >( m, &tn_mesh::laplace_tables, P, st ) )
     {
-        set_error( std::string( what ) + ": allocating the lateral quadrature table failed" );
+        set_error( std::string( what ) + ": allocating the lateral stencils failed" );
         return TN_ERR_NOMEM;
     }
-    P.radii = sizeof( T ) == 8 ? reinterpret_cast< const T* >( m->d_radii ) : reinterpret_cast< const T* >( m->d_radii32 );
-    P.k = k, P.mode_first = mode_first, P.mode_inner = mode_inner, P.mode_last = mode_last, P.single = single;
-    const long long cells  = (long long) kDiamonds * m->N * m->N * m->N;
-    const unsigned  blocks = unsigned( ( cells + 127 ) / 128 );
-    if ( k )
-        grad_cell_kernel< T, NC, true ><<< blocks, 128, 0, st >>>( P );
-    else
-        grad_cell_kernel< T, NC, false ><<< blocks, 128, 0, st >>>( P );
-    TN_LAUNCH_CHECK();
-    if ( comm_mode == TN_COMM_ADDITIVE )
-        return halo_sum< T >( m, dst, NC, st );
-    return TN_OK;
+    P.mode_first = mode_first, P.mode_inner = mode_inner, P.mode_last = mode_last;
+    return launch_lateral< LaplaceOp< T > >( m, P, nc, apply_mode, comm_mode, st );
 }
 
 // Laplace / DivKGrad coupling (laplace.hpp:140-168, div_k_grad.hpp:455-512):
@@ -390,7 +403,7 @@ int laplace_apply( const tn_mesh* m, int treat, int diag, int apply_mode, int co
     scalar_modes( m->N, treat, diag, f, i, l );
     const T* s[1] = { src };
     T*       d[1] = { dst };
-    return grad_family_apply< T, 1 >( m, nullptr, s, d, f, i, l, 0, apply_mode, comm_mode, st, "laplace_apply" );
+    return constant_gradient_apply< T >( m, 1, s, d, f, i, l, apply_mode, comm_mode, st, "laplace_apply" );
 }
 
 template < typename T >
@@ -398,11 +411,25 @@ int divkgrad_apply( const tn_mesh* m, const T* k, int treat, int diag, int singl
                     const T* src, T* dst, cudaStream_t st )
 {
     TN_CHECK_ARG( m && k && src && dst, "divkgrad_apply: null argument" );
-    int f, i, l;
-    scalar_modes( m->N, treat, diag, f, i, l );
-    const T* s[1] = { src };
-    T*       d[1] = { dst };
-    return grad_family_apply< T, 1 >( m, k, s, d, f, i, l, single != 0, apply_mode, comm_mode, st, "divkgrad_apply" );
+    TN_CHECK_ARG( apply_mode == TN_APPLY_REPLACE || apply_mode == TN_APPLY_ADD, "divkgrad_apply: bad apply mode" );
+    GradParams< T > P{};
+    scalar_modes( m->N, treat, diag, P.mode_first, P.mode_inner, P.mode_last );
+    if ( apply_mode == TN_APPLY_REPLACE )
+        TN_CUDA_TRY( cudaMemsetAsync( dst, 0, m->ns * sizeof( T ), st ) );
+    P.N = m->N, P.n1 = m->n1, P.geom = grad_geometry( m );
+    if ( !P.geom )
+    {
+        set_error( "divkgrad_apply: allocating the lateral quadrature table failed" );
+        return TN_ERR_NOMEM;
+    }
+    P.radii = sizeof( T ) == 8 ? reinterpret_cast< const T* >( m->d_radii ) : reinterpret_cast< const T* >( m->d_radii32 );
+    P.k = k, P.src = src, P.dst = dst, P.single = single != 0;
+    const long long cells = (long long) kDiamonds * m->N * m->N * m->N;
+    divkgrad_cell_kernel< T ><<< unsigned( ( cells + 127 ) / 128 ), 128, 0, st >>>( P );
+    TN_LAUNCH_CHECK();
+    if ( comm_mode == TN_COMM_ADDITIVE )
+        return halo_sum< T >( m, &dst, 1, st );
+    return TN_OK;
 }
 
 // VectorLaplace coupling (vector_laplace.hpp:181-210): the branch follows the
@@ -420,8 +447,8 @@ int vector_laplace_apply( const tn_mesh* m, int bc_cmb, int bc_surface, int diag
                   "vector_laplace_apply: boundary conditions must be Neumann or Dirichlet" );
     const int first = diag ? kDiag : ( bc_cmb == TN_BC_DIRICHLET ? kBot : kNeu );
     const int inner = diag ? kDiag : ( bc_surface == TN_BC_DIRICHLET ? kTop : kNeu );
-    return grad_family_apply< T, 3 >( m, nullptr, src, dst, first, inner, inner, 0, apply_mode, comm_mode, st,
-                                      "vector_laplace_apply" );
+    return constant_gradient_apply< T >( m, 3, src, dst, first, inner, inner, apply_mode, comm_mode, st,
+                                         "vector_laplace_apply" );
 }
 
 }  // namespace tn

@@ -326,7 +326,8 @@ int mesh_create_diamonds( const ShellTopology& t, double r_min, double r_max, in
             members.push_back( t.members[k] - lo );
         offsets.push_back( int( members.size() ) );
     }
-    m->n_halo_groups = int( offsets.size() ) - 1;
+    m->n_halo_groups  = int( offsets.size() ) - 1;
+    m->n_halo_members = int( members.size() );
     std::memcpy( m->penalty_gram_inv, t.gram_inv, sizeof( t.gram_inv ) );
 
     std::vector< int > lat_group( m->nlat, -1 );
@@ -397,6 +398,13 @@ extern "C" int tn_mesh_destroy( tn_mesh* m )
     cudaFree( m->d_lat_group );
     cudaFree( m->d_fv_ghost );
     cudaFree( m->d_fv_orient );
+    for ( tn_lateral_tables* t : { &m->laplace_tables, &m->mass_tables } )
+    {
+        cudaFree( t->lat );
+        cudaFree( t->rad );
+        cudaFree( t->lat32 );
+        cudaFree( t->rad32 );
+    }
     cudaFree( m->d_grad_geom );
     cudaFree( m->d_stokes_geom );
     cudaFree( m->d_red_partials );

@@ -1,0 +1,51 @@
+"""The separated form of the constant-coefficient operators (Laplace, VectorLaplace, mass matrix) against the oracle,
+copy by copy: every level whose block of 254 nodes ends inside a column or spans several, inputs whose duplicated
+nodes hold different values, and each apply / communication mode."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import rel
+from oracle_lib import Mesh
+
+pytestmark = pytest.mark.gpu
+
+
+def _apply(shell, C, pm, op_of, u, dtype, old, am, cm):
+    cls = shell.VectorQ1Vec if u.ndim == 5 else shell.VectorQ1Scalar
+    src, dst = cls(pm, dtype), cls(pm, dtype)
+    src.set_numpy(u)
+    dst.set_numpy(old)
+    shell.apply(op_of(am, cm), src, dst)
+    torch.cuda.synchronize()
+    return dst.numpy().reshape(u.shape).astype(np.float64)
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-13), (torch.float32, 1e-5)])
+@pytest.mark.parametrize("L", [1, 2, 3, 4, 5])
+@pytest.mark.parametrize("op,bc", [("laplace", 0), ("laplace", 1), ("vector", (0, 1)), ("vector", (1, 0)), ("mass", 0),
+                                   ("mass_diag", 0)])
+def test_every_copy_and_mode(op, bc, L, dtype, tol):
+    """FP32: 1e-5 is the tolerance of the other single-precision operator tests"""
+    from terraneo_b200 import shell, _capi as C
+    om, pm = Mesh(L), shell.ShellMesh(L)
+    rng = np.random.default_rng(L)
+    u = rng.normal(size=((3,) if op == "vector" else ()) + om.shape).astype(np.float32).astype(np.float64)
+    old = rng.normal(size=u.shape).astype(np.float32).astype(np.float64)
+    if op == "laplace":
+        ref, make = om.laplace(u, bc, 0), lambda am, cm: shell.Laplace(pm, bc, False, am, cm)
+    elif op == "vector":
+        ref, make = om.vector_laplace(u, *bc), lambda am, cm: shell.VectorLaplace(pm, *bc, False, am, cm)
+    else:
+        mode = int(op == "mass_diag")
+        ref, make = om.kmass(np.ones(om.shape), u, mode), lambda am, cm: shell.KMass(pm, None, mode, am, cm)
+
+    def halo(f):
+        return om.halo_sum(f).reshape(u.shape)
+
+    args = (shell, C, pm, make, u, dtype, old)
+    assert rel(_apply(*args, C.APPLY_REPLACE, C.COMM_ADDITIVE), ref.reshape(u.shape)) <= tol
+    own = _apply(*args, C.APPLY_REPLACE, C.COMM_SKIP)  # each copy its diamond's part: their sum is the result
+    assert rel(halo(own), ref.reshape(u.shape)) <= tol
+    assert rel(_apply(*args, C.APPLY_ADD, C.COMM_SKIP), own + old) <= tol
+    assert rel(_apply(*args, C.APPLY_ADD, C.COMM_ADDITIVE), halo(own + old)) <= tol
