@@ -139,6 +139,9 @@ struct tn_mesh
     uint8_t* d_fv_orient = nullptr;
 
     tn_lateral_tables laplace_tables, mass_tables;
+    // wedge vectors per triangle (cell.cuh), one allocation
+    double* d_triangles   = nullptr;
+    float*  d_triangles32 = nullptr;
 
     // lateral quadrature table of DivKGrad, built on first use:
     // [10][N][N][2 wedges][84]

@@ -15,6 +15,7 @@
 #include <map>
 #include <mutex>
 
+#include "cell.cuh"
 #include "common.cuh"
 
 namespace tn {
@@ -156,6 +157,74 @@ int halo_sum( const tn_mesh* m, T* const* fields, int nfields, cudaStream_t st )
 
 template int halo_sum< double >( const tn_mesh*, double* const*, int, cudaStream_t );
 template int halo_sum< float >( const tn_mesh*, float* const*, int, cudaStream_t );
+
+// a b - c d with the rounding error of c d put back (Kahan's difference of products: within 1.5 ulp)
+__device__ __forceinline__ double diff_of_products( double a, double b, double c, double d )
+{
+    const double cd = c * d, err = fma( -c, d, cd );
+    return fma( a, b, -cd ) + err;
+}
+
+// Thread per triangle: beta_1, beta_2, v, 1 / D and the radial and volume factors (cell.cuh).  Every layer of a column
+// uses the same entry, so its rounding does not average out: the cross products are formed to the last bits, and
+// D = v . p0 with the products' errors.
+template < typename T >
+__global__ void triangle_kernel( int N, size_t triangles, const double* __restrict__ coords,
+                                 const double* __restrict__ radii, T* table )
+{
+    const size_t t = blockIdx.x * size_t( blockDim.x ) + threadIdx.x;
+    if ( t >= triangles )
+        return;
+    const int     w = int( t & 1 ), y = int( t / 2 % N ), x = int( t / 2 / N % N ), d = int( t / 2 / N / N ), n1 = N + 1;
+    const double* p[3];
+    for ( int i = 0; i < 3; ++i )
+        p[i] = coords + lat_index( n1, d, x + wedge_node( w, i, 0 ), y + wedge_node( w, i, 1 ) ) * 3;
+    double a[3], b[3], q[kTriangle], D = 0.0, err = 0.0;
+    for ( int k = 0; k < 3; ++k )
+        a[k] = p[1][k] - p[0][k], b[k] = p[2][k] - p[0][k];
+    for ( int k = 0; k < 3; ++k )
+    {
+        const int i = ( k + 1 ) % 3, j = ( k + 2 ) % 3;
+        q[k]     = diff_of_products( b[i], p[0][j], b[j], p[0][i] );
+        q[3 + k] = diff_of_products( p[0][i], a[j], p[0][j], a[i] );
+        q[6 + k] = diff_of_products( a[i], b[j], a[j], b[i] );
+        const double pr = q[6 + k] * p[0][k], s = D + pr, z = s - D; // two-sum
+        err += fma( q[6 + k], p[0][k], -pr ) + ( ( D - ( s - z ) ) + ( pr - z ) );
+        D = s;
+    }
+    q[9] = 1.0 / ( D + err );
+    for ( int k = 0; k < kTriangle; ++k )
+        table[t * kTriangle + k] = T( q[k] );
+    // FV cells: the lateral factor of the inverse volume is 1 / (|D_0| + |D_1|), with the partner's D from its thread
+    const double other = __shfl_xor_sync( __activemask(), fabs( D + err ), 1 );
+    T*           fv    = table + triangles * kTriangle + 3 * N;
+    if ( w == 0 )
+        fv[t / 2] = T( 1.0 / ( fabs( D + err ) + other ) );
+    if ( t < size_t( N ) )
+    {
+        // h, r1 / h, r1 and the radial factor h / 2 (r(-g)^2 + r(g)^2) of the volume, g = 1 / sqrt(3)
+        const double r1 = radii[t], h = 0.5 * ( radii[t + 1] - r1 ), g = 0.5773502691896258;
+        const double rm = r1 + h * ( 1.0 - g ), rp = r1 + h * ( 1.0 + g );
+        table[triangles * kTriangle + t]         = T( h );
+        table[triangles * kTriangle + N + t]     = T( r1 / h );
+        table[triangles * kTriangle + 2 * N + t] = T( r1 );
+        fv[triangles / 2 + t]                    = T( 1.0 / ( 0.5 * h * ( rm * rm + rp * rp ) ) );
+    }
+}
+
+// both tables of cell.cuh, complete for every stream on return
+int build_triangle_tables( tn_mesh* m )
+{
+    const size_t   n = size_t( m->nd ) * m->N * m->N * 2, count = n * kTriangle + n / 2 + 4 * size_t( m->N );
+    const unsigned blocks = unsigned( ( n + 127 ) / 128 );
+    TN_CUDA_TRY( cudaMalloc( &m->d_triangles, count * ( sizeof( double ) + sizeof( float ) ) ) );
+    m->d_triangles32 = reinterpret_cast< float* >( m->d_triangles + count );
+    triangle_kernel< double ><<< blocks, 128 >>>( m->N, n, m->d_coords, m->d_radii, m->d_triangles );
+    triangle_kernel< float ><<< blocks, 128 >>>( m->N, n, m->d_coords, m->d_radii, m->d_triangles32 );
+    TN_LAUNCH_CHECK();
+    TN_CUDA_TRY( cudaStreamSynchronize( nullptr ) );
+    return TN_OK;
+}
 
 }  // namespace tn
 
@@ -349,7 +418,7 @@ int mesh_create_diamonds( const ShellTopology& t, double r_min, double r_max, in
          ( rc = upload( offsets.data(), offsets.size(), &m->d_halo_offsets ) ) ||
          ( nd == kDiamonds && ( rc = upload( t.fv_ghost.data(), t.fv_ghost.size(), &m->d_fv_ghost ) ) ) ||
          ( rc = upload( members.data(), members.size(), &m->d_halo_members ) ) ||
-         ( rc = upload( lat_group.data(), lat_group.size(), &m->d_lat_group ) ) )
+         ( rc = upload( lat_group.data(), lat_group.size(), &m->d_lat_group ) ) || ( rc = build_triangle_tables( m ) ) )
     {
         tn_mesh_destroy( m );
         return rc;
@@ -405,6 +474,7 @@ extern "C" int tn_mesh_destroy( tn_mesh* m )
         cudaFree( t->lat32 );
         cudaFree( t->rad32 );
     }
+    cudaFree( m->d_triangles );
     cudaFree( m->d_grad_geom );
     cudaFree( m->d_stokes_geom );
     cudaFree( m->d_red_partials );

@@ -1,0 +1,128 @@
+"""The kernels that run one thread per cell with the upper nodes handed to the lane above (cell.cuh), against the oracle
+at the levels where that can go wrong: partial warps and several columns per warp (1-3), one column per warp (5), a
+column over two warps (6); and the two-kernel CG (lateral_cg.cuh) against the oracle's iterates."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import random_vector, rel, viscosity_field
+from oracle_lib import Mesh, pcg
+
+pytestmark = pytest.mark.gpu
+LEVELS = [1, 2, 3, 5, 6]
+TOL = {torch.float64: 1e-12, torch.float32: 1e-5}  # the tolerances of the operators' other tests
+
+
+def _run(shell, op, pm, u, dtype, out_mesh=None, ncomp=None):
+    cls = {1: shell.VectorQ1Scalar, 3: shell.VectorQ1Vec}
+    src = cls[3 if u.ndim == 5 else 1](pm if op is None or u.shape[-1] == pm.n1 else out_mesh, dtype)
+    dst = cls[ncomp or src.ncomp](out_mesh or pm, dtype)
+    src.set_numpy(u)
+    shell.apply(op, src, dst)
+    torch.cuda.synchronize()
+    return dst.numpy().reshape((3,) + dst.mesh.shape if dst.ncomp == 3 else dst.mesh.shape).astype(np.float64)
+
+
+@pytest.fixture(scope="module", params=LEVELS)
+def case(request):
+    from terraneo_b200 import shell
+    L = request.param
+    om = Mesh(L)
+    return L, om, shell.ShellMesh(L), viscosity_field(om, seed=L), random_vector(om, seed=L)
+
+
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+@pytest.mark.parametrize("treat", [True, False])
+def test_divkgrad(case, treat, dtype):
+    from terraneo_b200 import shell
+    L, om, pm, k, u = case
+    kv = shell.VectorQ1Scalar(pm, dtype)
+    kv.set_numpy(k)
+    for single in (False, True) if L < 6 else (False,):
+        got = _run(shell, shell.DivKGrad(pm, kv, treat, single_quadpoint=single), pm, u[0], dtype)
+        assert rel(got, om.divkgrad(k, u[0], treat, False, single)) <= TOL[dtype]
+
+
+@pytest.mark.parametrize("treat", [True, False])
+def test_epsdivdiv3x2(case, treat):
+    from terraneo_b200 import shell
+    L, om, pm, k, u = case
+    kv = shell.VectorQ1Scalar(pm)
+    kv.set_numpy(k)
+    assert rel(_run(shell, shell.EpsilonDivDiv(pm, kv, treat), pm, u, torch.float64),
+               om.epsdivdiv3x2(k, u, treat)) <= 1e-12
+
+
+@pytest.mark.parametrize("kappa,treat,lumped", [(1e-3, True, False), (1e-6, False, False), (0.5, True, True),
+                                                (0.0, True, False)])
+def test_supg(case, kappa, treat, lumped):
+    """Peclet numbers from 1e-3 (the small-argument branch of tau) to 1e7; some nodes at rest"""
+    from terraneo_b200 import shell
+    L, om, pm, k, u = case
+    if L == 6 and kappa != 1e-3:
+        return
+    vel = np.where(np.abs(u[:1]) > 1.5, 0.0, u)
+    vv = shell.VectorQ1Vec(pm)
+    vv.set_numpy(vel)
+    op = shell.UnsteadyAdvectionDiffusionSUPG(pm, vv, kappa, 1e-2, treat, False, 1.5, lumped)
+    assert rel(_run(shell, op, pm, u[0], torch.float64), om.supg(vel, u[0], kappa, 1e-2, 1.5, lumped, treat)) <= 1e-12
+
+
+@pytest.mark.parametrize("bc", [(1, 2), (2, 0)])
+def test_stokes_blocks(case, bc):
+    from terraneo_b200 import shell
+    L, om, pm, k, u = case
+    if L < 2:
+        return
+    oc, pc = Mesh(L - 1), shell.ShellMesh(L - 1)
+    assert rel(_run(shell, shell.Divergence(pm, pc, *bc), pm, u, torch.float64, pc, 1),
+               om.divergence(oc, u, *bc)) <= 1e-12
+    p = random_vector(oc, seed=1, ncomp=1)
+    vp, vu = shell.VectorQ1Scalar(pc), shell.VectorQ1Vec(pm)
+    vp.set_numpy(p)
+    shell.apply(shell.Gradient(pm, pc, *bc), vp, vu)
+    assert rel(vu.numpy(), om.gradient(oc, p, *bc)) <= 1e-12
+
+
+@pytest.mark.parametrize("bc", [(0, 0), (1, 2), (2, 0)])
+def test_viscosity_gradient(case, bc):
+    """linear in k: d(lambda^T A(k) u)/dk times a perturbation of k, summed over the owned nodes, is lambda^T A(dk) u"""
+    from terraneo_b200 import shell
+    L, om, pm, k, u = case
+    if L > 5:
+        return
+    lam, dk = random_vector(om, seed=L + 1), random_vector(om, seed=L + 2, ncomp=1)
+    vu, vl, g = shell.VectorQ1Vec(pm), shell.VectorQ1Vec(pm), shell.VectorQ1Scalar(pm)
+    vu.set_numpy(u)
+    vl.set_numpy(lam)
+    shell.epsdivdiv_kgrad(pm, *bc, vu, vl, g)
+    own = om.omask == 1
+    terms = om.kerngen(dk, u, *bc) * lam
+    want = float((terms * own).sum())
+    # a sum of N terms of both signs: bounded by their absolute sum
+    assert abs(float((g.numpy()[0] * dk * own).sum()) - want) <= 1e-12 * float(np.abs(terms * own).sum())
+
+
+@pytest.mark.parametrize("its", [1, 2, 9, 17])
+def test_cg_iterates(case, its):
+    """the iterate after 1, 2 (each direction field), 9 and 17 (the stopping flag is looked at every 8) steps"""
+    from terraneo_b200 import shell
+    L, om, pm, k, u = case
+    if L > 3:
+        return
+    b = om.kmass(np.ones(om.shape), u[0], 0)
+    b[..., 0] = b[..., -1] = 0.0
+    vb, vx = shell.VectorQ1Scalar(pm), shell.VectorQ1Scalar(pm)
+    vb.set_numpy(b)
+    n, rr = shell.laplace_pcg(pm, vb, vx, its, 1e-11)
+    want, m = om.laplace_pcg(b, its, 1e-11)
+    assert abs(n - m) <= 1 and rel(vx.numpy()[0], want) <= 1e-11  # level 1 ends by exhausting its few directions
+    fv = np.zeros(om.fv_shape)
+    fv[:, 1:-1, 1:-1, 1:-1] = np.random.default_rng(its).normal(size=(10,) + (om.N,) * 3)
+    n = shell.l2_project_fv_to_fe(pm, torch.as_tensor(fv, device="cuda"), vx, max_iterations=its)
+    rhs, _ = om.fv_to_fe_rhs(fv)
+    ones = np.ones(om.shape)
+    # from x: the projection solves for the correction of its initial guess
+    r0 = rhs - om.kmass(ones, want, 0)
+    dx, m = pcg(lambda v: om.kmass(ones, v, 0), om.dot, r0, its, 1e-12, 1e-12)
+    assert abs(n - m) <= 1 and rel(vx.numpy()[0], want + dx) <= 1e-11
