@@ -143,10 +143,7 @@ struct tn_mesh
     double* d_triangles   = nullptr;
     float*  d_triangles32 = nullptr;
 
-    // lateral quadrature table of DivKGrad, built on first use:
-    // [10][N][N][2 wedges][84]
-    std::mutex      geom_mutex;
-    double*         d_grad_geom = nullptr;
+    std::mutex      geom_mutex; // guards the tables built on first use
     double*         d_stokes_geom = nullptr; // Divergence / Gradient, this mesh as the velocity mesh
 
     // fs/fs penalty: the orthonormalised modes are m = C (e_j x x); G = C^T C

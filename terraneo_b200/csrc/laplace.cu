@@ -9,6 +9,7 @@
 // diagonal, as selected per operator below.
 #include <cmath>
 
+#include "cell.cuh"
 #include "common.cuh"
 #include "lateral.cuh"
 #include "wedge.cuh"
@@ -17,185 +18,199 @@ namespace tn {
 
 namespace {
 
-__device__ __constant__ const double kQP32[3][2] = { { 0.6666666666666666, 0.1666666666666667 },
-                                                     { 0.1666666666666667, 0.6666666666666666 },
-                                                     { 0.1666666666666667, 0.1666666666666667 } };
-constexpr double kQP32Host[3][2] = { { 0.6666666666666666, 0.1666666666666667 },
-                                     { 0.1666666666666667, 0.6666666666666666 },
-                                     { 0.1666666666666667, 0.1666666666666667 } };
-constexpr double kZeta32 = 0.5773502691896257;
-constexpr double kW32    = 0.1666666666666667;
-
 template < typename T >
-struct GradParams
+struct DivKGradParams
 {
-    int             N, n1;
-    const double*   geom; // lateral quadrature table, kGeomStride doubles per wedge
-    const T*        radii;
-    const T*        k; // nodal coefficient
-    const T*        src;
-    T*              dst;
-    int             mode_first, mode_inner, mode_last; // coupling of layer 0, 1..N-2, N-1
-    int             single;                            // 1-point rule instead of 3x2
+    int      N, n1;
+    const T* table;
+    const T* k; // nodal coefficient
+    const T* src;
+    T*       dst;
+    int      treat, single;
+    unsigned cell_blocks; // blocks of cells; those after them add diagonals
 };
 
-// Factored wedge stiffness.  For x = r(zeta) ((1-xi-eta) p0 + xi p1 + eta p2)
-// with a = p1 - p0, b = p2 - p0, v = a x b, c = p0 + xi a + eta b and
-// h = (r2 - r1) / 2, the Jacobian columns are r a, r b, h c, so
-// |det J| = r^2 h |D| with D = v . p0 (constant on the wedge) and the
-// physical gradient of the shape function of node n (lateral vertex m, side
-// sign s_n = -+1/2, radial factor nr_n(zeta) = (1 -+ zeta)/2) is
-//     g_n = ( nr_n / r u_m + s_n lat_m / h v ) / D,
-//     u_1 = b x c, u_2 = c x a, u_0 = -(u_1 + u_2).
-// A quadrature point's contribution w |det J| g_i . g_j therefore splits into
-// lateral factors (u_m . u_m', lat_m lat_m' |v|^2, (u_m . v) lat_m', all
-// / |D|) times radial ones (h nr_i nr_j, r^2 / h, r nr), and on the
-// tensor-product 3x2 rule the lateral and radial sums separate: with a
-// constant coefficient (Laplace, VectorLaplace) the whole operator is a sum of
-// lateral stencils times radial factors (LaplaceOp, lateral.cuh).  DivKGrad's
-// nodal k keeps the points apart: the lateral factors depend only on the
-// triangle, so they are tabulated once per mesh, sets 0-2 for the three
-// lateral points of the 3x2 rule and set 3 for the centroid (weights applied
-// in the kernel).  Each set is U (6, symmetric), Lam (6, symmetric), W (9,
-// row-major).  Mathematically the same stiffness as the per-point Jacobian of
-// fe/wedge/integrands.hpp, evaluated with far fewer operations.
-constexpr int kGeomSet    = 21;
-constexpr int kGeomStride = 4 * kGeomSet;
-
-// radial factors of one set: R[li + lj] (bottom/top node pairs), S2, P[l]
-template < typename T >
-struct Radial
+// One wedge of DivKGrad from the values s of its nodes and k there; out[n] = its
+// row of node n.  In the factored form of cell.cuh the scaled gradient of u is
+// beta_1 S_1 + beta_2 S_2 + v Z with edge differences S_i that depend on zeta only
+// and Z = rho T - xi S_1 - eta S_2, so a point needs Z and its product with v,
+// and the rows follow from the zeta's summed flux against beta_1, beta_2 and the
+// moments of (flux . v) over the points, all through the six scalar products of
+// beta_1, beta_2, v: about 150 multiply-adds per wedge (470 when the symmetric
+// 6 x 6 matrix is formed from a table of 63 lateral factors per wedge).
+// Apply with its halo, FP64: 330 -> 96 us at level 6, 2,562 -> 675 us at level 7;
+// bound by instruction issue (56 % of the slots).
+template < typename T, bool SINGLE >
+__device__ __forceinline__ void divkgrad_wedge( const Triangle< T >& G, T h, T rho_m, const T ( &s )[6], const T ( &kn )[6],
+                                                T ( &out )[6] )
 {
-    T R[3], S2, P[2];
-};
-
-template < typename T >
-__device__ __forceinline__ void add_set( T A[21], const double* __restrict__ G, const Radial< T >& f )
-{
-    T U[3][3], Lm[3][3], W[3][3];
-    U[0][0] = T( G[0] ), U[0][1] = U[1][0] = T( G[1] ), U[0][2] = U[2][0] = T( G[2] );
-    U[1][1] = T( G[3] ), U[1][2] = U[2][1] = T( G[4] ), U[2][2] = T( G[5] );
-    Lm[0][0] = T( G[6] ), Lm[0][1] = Lm[1][0] = T( G[7] ), Lm[0][2] = Lm[2][0] = T( G[8] );
-    Lm[1][1] = T( G[9] ), Lm[1][2] = Lm[2][1] = T( G[10] ), Lm[2][2] = T( G[11] );
-#pragma unroll
-    for ( int i = 0; i < 9; ++i )
-        ( &W[0][0] )[i] = T( G[12 + i] );
-    int e = 0;
-#pragma unroll
-    for ( int i = 0; i < 6; ++i )
-#pragma unroll
-        for ( int j = i; j < 6; ++j )
-        {
-            const int li = i / 3, lj = j / 3, mi = i % 3, mj = j % 3;
-            const T   si = li ? T( 0.5 ) : T( -0.5 ), sj = lj ? T( 0.5 ) : T( -0.5 );
-            A[e++] += f.R[li + lj] * U[mi][mj] + ( si * sj ) * f.S2 * Lm[mi][mj] + sj * f.P[li] * W[mi][mj] +
-                      si * f.P[lj] * W[mj][mi];
-        }
-}
-
-__host__ __device__ constexpr int sym6( int i, int j )
-{
-    return i <= j ? 6 * i - i * ( i - 1 ) / 2 + j - i : 6 * j - j * ( j - 1 ) / 2 + i - j;
-}
-
-// One thread per cell (r fastest: neighbouring threads share the lateral
-// table entry and touch consecutive addresses).  Each wedge's symmetric 6x6
-// matrix is formed from its table entry and the layer's radial factors; the 8
-// node sums of the cell are kept in registers and added with one atomic each.
-template < typename T >
-__global__ void __launch_bounds__( 128 ) divkgrad_cell_kernel( GradParams< T > P )
-{
-    const int       N = P.N, n1 = P.n1;
-    const long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x;
-    if ( t >= (long long) kDiamonds * N * N * N )
-        return;
-    const int r = int( t % N );
-    const int y = int( ( t / N ) % N );
-    const int x = int( ( t / ( (long long) N * N ) ) % N );
-    const int d = int( t / ( (long long) N * N * N ) );
-
-    const int mode = layer_mode( r, N, P.mode_first, P.mode_inner, P.mode_last );
-    const T   r1 = P.radii[d * n1 + r], r2 = P.radii[d * n1 + r + 1];
-    const T   h = T( 0.5 ) * ( r2 - r1 );
-    bool      cpl[6];
+    const T b11 = dot3( G.b1, G.b1 ), b12 = dot3( G.b1, G.b2 ), b22 = dot3( G.b2, G.b2 );
+    const T a1 = dot3( G.b1, G.v ), a2 = dot3( G.b2, G.v ), vv = dot3( G.v, G.v );
+    const T t[3] = { T( 0.5 ) * ( s[3] - s[0] ), T( 0.5 ) * ( s[4] - s[1] ), T( 0.5 ) * ( s[5] - s[2] ) };
+    const T e1b = s[1] - s[0], e2b = s[2] - s[0], e1t = s[4] - s[3], e2t = s[5] - s[3];
+    T       L[3] = { T( 0 ), T( 0 ), T( 0 ) };
 #pragma unroll
     for ( int n = 0; n < 6; ++n )
-        cpl[n] = mode == kNeu || ( mode == kBot && n >= 3 ) || ( mode == kTop && n < 3 );
-
-    T out[2][2][2];
-    for ( int i = 0; i < 8; ++i )
-        ( &out[0][0][0] )[i] = T( 0 );
-#pragma unroll
-    for ( int w = 0; w < 2; ++w )
+        out[n] = T( 0 );
+    if ( SINGLE )
     {
-        const double* G = P.geom + ( ( ( size_t( d ) * N + x ) * N + y ) * 2 + w ) * kGeomStride;
-        T             s[6], kv[6];
+        // quad_felippa_1x1: (1/3, 1/3, 0), weight 1; k at the centroid is the mean of the six
+        const T w  = ( kn[0] + kn[1] + kn[2] + kn[3] + kn[4] + kn[5] ) * T( 1.0 / 6.0 ) * h * fabs( G.iD );
+        const T S1 = T( 0.5 ) * ( e1b + e1t ), S2 = T( 0.5 ) * ( e2b + e2t );
+        const T Z  = ( rho_m * ( t[0] + t[1] + t[2] ) - S1 - S2 ) * T( 1.0 / 3.0 );
+        const T x  = w * ( a1 * S1 + a2 * S2 + vv * Z ) * T( 1.0 / 3.0 );
+        const T f1 = w * ( b11 * S1 + b12 * S2 + a1 * Z ) - x, f2 = w * ( b12 * S1 + b22 * S2 + a2 * Z ) - x;
+        out[0] = out[3] = T( -0.5 ) * ( f1 + f2 ), out[1] = out[4] = T( 0.5 ) * f1, out[2] = out[5] = T( 0.5 ) * f2;
+        L[0] = L[1] = L[2] = rho_m * x;
+    }
+    else
+    {
+        // omega = k h / (6 |D|) at the lateral points, bottom and top: k there is (the sum + 3 the near vertex) / 6, and both
+        // sixths are one rounded factor
+        const T scale = T( 1.0 / 36.0 ) * h * fabs( G.iD );
+        const T sb = kn[0] + kn[1] + kn[2], st = kn[3] + kn[4] + kn[5];
+        const T ts = ( t[0] + t[1] + t[2] ) * T( 1.0 / 6.0 );
 #pragma unroll
-        for ( int n = 0; n < 6; ++n )
+        for ( int zq = 0; zq < 2; ++zq )
         {
-            const size_t i = lat_index( n1, d, x + kWedgeNode[w][n][0], y + kWedgeNode[w][n][1] ) * n1 + r +
-                             kWedgeNode[w][n][2];
-            s[n]  = P.src[i];
-            kv[n] = P.k[i];
-        }
-        T A[21];
-#pragma unroll
-        for ( int e = 0; e < 21; ++e )
-            A[e] = T( 0 );
-        if ( P.single )
-        {
-            // quad_felippa_1x1: (1/3, 1/3, 0), weight 1; k at the centroid is the mean of the six
-            const T    ke = ( kv[0] + kv[1] + kv[2] + kv[3] + kv[4] + kv[5] ) * T( 1.0 / 6.0 );
-            const T    rm = r1 + h;
-            Radial< T > f;
-            f.R[0] = f.R[1] = f.R[2] = ke * h * T( 0.25 );
-            f.S2                     = ke * rm * rm / h;
-            f.P[0] = f.P[1] = ke * rm * T( 0.5 );
-            add_set( A, G + 3 * kGeomSet, f );
-        }
-        else
-        {
+            const T nb = T( zq ? 0.5 * ( 1.0 - kFelippaZ ) : 0.5 * ( 1.0 + kFelippaZ ) );
+            const T nt = T( zq ? 0.5 * ( 1.0 + kFelippaZ ) : 0.5 * ( 1.0 - kFelippaZ ) );
+            const T rho = rho_m + T( zq ? kFelippaZ : -kFelippaZ );
+            const T S1 = nb * e1b + nt * e1t, S2 = nb * e2b + nt * e2t;
+            const T Z0 = rho * ts - T( 1.0 / 6.0 ) * ( S1 + S2 ), pv = a1 * S1 + a2 * S2;
+            T       om = T( 0 ), Zs = T( 0 ), ev[2];
 #pragma unroll
             for ( int q = 0; q < 3; ++q )
             {
-                const T lat[3] = { T( 1.0 - kQP32[q][0] - kQP32[q][1] ), T( kQP32[q][0] ), T( kQP32[q][1] ) };
-                const T kb = lat[0] * kv[0] + lat[1] * kv[1] + lat[2] * kv[2];
-                const T kt = lat[0] * kv[3] + lat[1] * kv[4] + lat[2] * kv[5];
-                Radial< T > f{};
-#pragma unroll
-                for ( int zq = 0; zq < 2; ++zq )
-                {
-                    const T zeta = zq ? T( kZeta32 ) : T( -kZeta32 );
-                    const T nb = T( 0.5 ) * ( T( 1 ) - zeta ), nt = T( 0.5 ) * ( T( 1 ) + zeta );
-                    const T rr = r1 + h * ( T( 1 ) + zeta );
-                    const T wk = T( kW32 ) * ( nb * kb + nt * kt );
-                    f.R[0] += wk * h * nb * nb, f.R[1] += wk * h * nb * nt, f.R[2] += wk * h * nt * nt;
-                    f.S2 += wk * rr * rr / h;
-                    f.P[0] += wk * rr * nb, f.P[1] += wk * rr * nt;
-                }
-                add_set( A, G + q * kGeomSet, f );
+                const int m = ( q + 1 ) % 3; // point q lies next to vertex m
+                const T   w = scale * ( nb * ( sb + T( 3 ) * kn[m] ) + nt * ( st + T( 3 ) * kn[3 + m] ) );
+                const T   Z = Z0 + T( 0.5 ) * ( q == 0 ? rho * t[1] - S1 : ( q == 1 ? rho * t[2] - S2 : rho * t[0] ) );
+                om += w;
+                Zs += w * Z;
+                if ( q < 2 )
+                    ev[q] = w * ( pv + vv * Z );
             }
-        }
-        T sc[6];
-#pragma unroll
-        for ( int n = 0; n < 6; ++n )
-            sc[n] = cpl[n] ? s[n] : T( 0 );
-#pragma unroll
-        for ( int i = 0; i < 6; ++i )
-        {
-            T acc = T( 0 );
-#pragma unroll
-            for ( int j = 0; j < 6; ++j )
-                acc += A[sym6( i, j )] * sc[j];
-            if ( !cpl[i] )
-                acc = A[sym6( i, i )] * s[i];
-            out[kWedgeNode[w][i][0]][kWedgeNode[w][i][1]][kWedgeNode[w][i][2]] += acc;
+            // flux . v summed over the points and its moments with xi and eta
+            const T V = om * pv + vv * Zs, X = T( 1.0 / 6.0 ) * V + T( 0.5 ) * ev[0], Y = T( 1.0 / 6.0 ) * V + T( 0.5 ) * ev[1];
+            const T f1 = om * ( b11 * S1 + b12 * S2 ) + a1 * Zs - X, f2 = om * ( b12 * S1 + b22 * S2 ) + a2 * Zs - Y;
+            const T f0 = -( f1 + f2 );
+            out[0] += nb * f0, out[1] += nb * f1, out[2] += nb * f2;
+            out[3] += nt * f0, out[4] += nt * f1, out[5] += nt * f2;
+            L[0] += rho * ( V - X - Y ), L[1] += rho * X, L[2] += rho * Y;
         }
     }
-    for ( int dx = 0; dx < 2; ++dx )
-        for ( int dy = 0; dy < 2; ++dy )
-            for ( int dz = 0; dz < 2; ++dz )
-                atomicAdd( P.dst + lat_index( n1, d, x + dx, y + dy ) * n1 + r + dz, out[dx][dy][dz] );
+#pragma unroll
+    for ( int m = 0; m < 3; ++m )
+        out[m] -= T( 0.5 ) * L[m], out[3 + m] += T( 0.5 ) * L[m];
+}
+
+// adds the diagonal entries of the three lower (top false) or upper nodes of a wedge times their values
+template < typename T >
+__device__ __forceinline__ void divkgrad_diagonal( const DivKGradParams< T >& P, int d, int x, int y, int r, int w, bool top )
+{
+    const T             h = layer_h( P.table, P.N, r ), rq = layer_q( P.table, P.N, r ), side = top ? T( 1 ) : T( -1 );
+    const Triangle< T > G( P.table, P.N, d, x, y, w );
+    unsigned            node[4], id[3];
+    T                   kn[6], o[3] = { T( 0 ), T( 0 ), T( 0 ) };
+    cell_nodes( P.n1, d, x, y, r, node );
+    wedge_columns( node, w, id );
+#pragma unroll
+    for ( int n = 0; n < 6; ++n )
+        kn[n] = P.k[id[n % 3] + n / 3];
+    for ( int q = 0; q < ( P.single ? 1 : 6 ); ++q )
+    {
+        const T xi = P.single ? T( 1.0 / 3.0 ) : T( felippa_xi( q ) ), eta = P.single ? T( 1.0 / 3.0 ) : T( felippa_eta( q ) );
+        const T zeta   = P.single ? T( 0 ) : T( q < 3 ? -kFelippaZ : kFelippaZ );
+        const T lat[3] = { T( 1 ) - xi - eta, xi, eta };
+        T       k      = T( 0 );
+#pragma unroll
+        for ( int n = 0; n < 6; ++n )
+            k += lat[n % 3] * T( 0.5 ) * ( n < 3 ? T( 1 ) - zeta : T( 1 ) + zeta ) * kn[n];
+        const T om = ( P.single ? T( 1 ) : T( kFelippaW ) ) * k * h * fabs( G.iD ), rho = rq + T( 1 ) + zeta;
+#pragma unroll
+        for ( int m = 0; m < 3; ++m )
+        {
+            T g[3];
+            scaled_gradient( G, m, side, xi, eta, zeta, rho, g );
+            o[m] += om * dot3( g, g );
+        }
+    }
+#pragma unroll
+    for ( int m = 0; m < 3; ++m )
+        atomicAdd( P.dst + id[m] + top, o[m] * P.src[id[m] + top] );
+}
+
+// One thread per cell (r fastest), contributions added by add_column.  With the
+// boundary treatment the CMB nodes of layer 0 (otherwise the SURFACE nodes of
+// layer N - 1) enter with zero and keep their diagonal, which further blocks of the
+// launch add (one thread per lateral cell, wedge and side).
+template < typename T, bool SINGLE >
+__global__ void __launch_bounds__( 128, 4 ) divkgrad_kernel( DivKGradParams< T > P )
+{
+    const int N = P.N, n1 = P.n1;
+    int       d, x, y, r;
+    if ( blockIdx.x >= P.cell_blocks )
+    {
+        int  w;
+        bool top;
+        if ( boundary_item( ( blockIdx.x - P.cell_blocks ) * blockDim.x + threadIdx.x, N, d, x, y, r, w, top ) )
+            divkgrad_diagonal( P, d, x, y, r, w, top );
+        return;
+    }
+    const bool in  = cell_of( blockIdx.x * (long long) blockDim.x + threadIdx.x, N, d, x, y, r );
+    const bool bot = P.treat && r == 0, top = P.treat && !bot && r == N - 1;
+    const T    h = layer_h( P.table, N, r ), rho_m = layer_q( P.table, N, r ) + T( 1 );
+    T* const   dst[1] = { P.dst };
+    unsigned   node[4];
+    T          s[4][2], k[4][2], acc[2][2];
+    cell_nodes( n1, d, x, y, r, node );
+#pragma unroll
+    for ( int i = 0; i < 4; ++i )
+    {
+#pragma unroll
+        for ( int l = 0; l < 2; ++l )
+        {
+            const T v = P.src[node[i] + l];
+            s[i][l]   = ( l ? top : bot ) ? T( 0 ) : v;
+            k[i][l]   = P.k[node[i] + l];
+        }
+    }
+#pragma unroll
+    for ( int w = 0; w < 2; ++w )
+    {
+        const Triangle< T > G( P.table, N, d, x, y, w );
+        T                   sw[6], kw[6], out[6];
+#pragma unroll
+        for ( int n = 0; n < 6; ++n )
+        {
+            const int i = wedge_node( w, n, 0 ) + 2 * wedge_node( w, n, 1 );
+            sw[n] = s[i][n / 3], kw[n] = k[i][n / 3];
+        }
+        divkgrad_wedge< T, SINGLE >( G, h, rho_m, sw, kw, out );
+        const T low0[1] = { out[0] }, high0[1] = { out[3] };
+        add_column< T, 1 >( dst, node[w ? 3 : 0], r, N, in, !bot, !top, low0, high0 );
+#pragma unroll
+        for ( int m = 1; m < 3; ++m )
+        {
+            const int a = w ? 2 - m : m - 1; // vertex m of wedge 0 is vertex 3 - m of wedge 1
+            if ( w == 0 )
+                acc[a][0] = out[m], acc[a][1] = out[3 + m];
+            else
+            {
+                const T low[1] = { acc[a][0] + out[m] }, high[1] = { acc[a][1] + out[3 + m] };
+                add_column< T, 1 >( dst, node[3 - m], r, N, in, !bot, !top, low, high );
+            }
+        }
+    }
+}
+
+// the diagonal alone: one thread per cell, wedge and side (blockIdx.y)
+template < typename T >
+__global__ void __launch_bounds__( 128 ) divkgrad_diagonal_kernel( DivKGradParams< T > P )
+{
+    int d, x, y, r;
+    if ( cell_of( blockIdx.x * (long long) blockDim.x + threadIdx.x, P.N, d, x, y, r ) )
+        divkgrad_diagonal( P, d, x, y, r, int( blockIdx.y & 1 ), blockIdx.y >= 2 );
 }
 
 // The lateral factors of a triangle at a lateral point with sig = 1 / |D|: u[3] and lat[3] (factored stiffness
@@ -234,10 +249,11 @@ struct LateralTriangle
 // the stencils U, W^T (per level; rows sum to zero because sum_m u_m = 0) and
 // Lam, W (on the difference of the levels), all summed over the 3x2 rule's
 // lateral points with weight 1/6, and its radial factors R[0] = R[2], R[1],
-// S2 / 4, P[0] / 2, P[1] / 2: add_set's entries, both rows sharing the differences.
+// S2 / 4, P[0] / 2, P[1] / 2 (R = h sum nr nr, S2 = sum r^2 / h, P = sum r nr),
+// both rows sharing the differences.
 // Apply with its halo, FP64, before (one thread per cell, atomics) and now:
-// Laplace 112 -> 39 us at level 6, 911 -> 271 us at level 7 (1.3 TB/s of its
-// 16 bytes per node); VectorLaplace 228 -> 118 us at level 6; FP32 Laplace
+// Laplace 112 -> 33 us at level 6, 911 -> 226 us at level 7 (1.5 TB/s of its
+// 16 bytes per node); VectorLaplace 228 -> 99 us at level 6; FP32 Laplace
 // 84 -> 25 us at level 6.
 template < typename T >
 struct LaplaceOp
@@ -275,8 +291,8 @@ struct LaplaceOp
         for ( int q = 0; q < 3; ++q )
         {
             double u[3][3], l[3];
-            tri.at( kQP32[q][0], kQP32[q][1], u, l );
-            const double f = kW32 * tri.sig;
+            tri.at( felippa_xi( q ), felippa_eta( q ), u, l );
+            const double f = kFelippaW * tri.sig;
             A[0] += f * LateralTriangle::dot( u[i], u[j] );
             A[1] += f * LateralTriangle::dot( u[j], tri.v ) * l[i];
             A[2] += f * l[i] * l[j] * vv;
@@ -290,73 +306,13 @@ struct LaplaceOp
             f[k] = 0.0;
         for ( int zq = 0; zq < 2; ++zq )
         {
-            const double zeta = zq ? kZeta32 : -kZeta32, nb = 0.5 * ( 1.0 - zeta ), nt = 0.5 * ( 1.0 + zeta );
+            const double zeta = zq ? kFelippaZ : -kFelippaZ, nb = 0.5 * ( 1.0 - zeta ), nt = 0.5 * ( 1.0 + zeta );
             const double rr   = r1 + h * ( 1.0 + zeta );
             f[0] += h * nb * nb, f[1] += h * nb * nt, f[2] += 0.25 * rr * rr / h;
             f[3] += 0.5 * rr * nb, f[4] += 0.5 * rr * nt;
         }
     }
 };
-
-// Host tabulation of DivKGrad's lateral factors (double), one entry per wedge.
-void build_grad_geometry( const tn_mesh* m, std::vector< double >& G )
-{
-    const int    N = m->N, n1 = m->n1;
-    const int    wn[2][3][2] = { { { 0, 0 }, { 1, 0 }, { 0, 1 } }, { { 1, 1 }, { 0, 1 }, { 1, 0 } } };
-    const double pts[4][2]   = { { kQP32Host[0][0], kQP32Host[0][1] },
-                                 { kQP32Host[1][0], kQP32Host[1][1] },
-                                 { kQP32Host[2][0], kQP32Host[2][1] },
-                                 { 1.0 / 3.0, 1.0 / 3.0 } };
-    G.assign( size_t( kDiamonds ) * N * N * 2 * kGeomStride, 0.0 );
-    for ( int d = 0; d < kDiamonds; ++d )
-        for ( int x = 0; x < N; ++x )
-            for ( int y = 0; y < N; ++y )
-                for ( int w = 0; w < 2; ++w )
-                {
-                    double* g = G.data() + ( ( ( size_t( d ) * N + x ) * N + y ) * 2 + w ) * kGeomStride;
-                    const double* p[3];
-                    for ( int k = 0; k < 3; ++k )
-                        p[k] = m->h_coords.data() + lat_index( n1, d, x + wn[w][k][0], y + wn[w][k][1] ) * 3;
-                    const LateralTriangle tri( p[0], p[1], p[2] );
-                    const double   vv = LateralTriangle::dot( tri.v, tri.v );
-                    for ( int q = 0; q < 4; ++q )
-                    {
-                        double u[3][3], lat[3];
-                        tri.at( pts[q][0], pts[q][1], u, lat );
-                        double* set = g + q * kGeomSet;
-                        for ( int i = 0; i < 3; ++i )
-                            for ( int j = i; j < 3; ++j )
-                                *set++ = tri.sig * LateralTriangle::dot( u[i], u[j] );
-                        for ( int i = 0; i < 3; ++i )
-                            for ( int j = i; j < 3; ++j )
-                                *set++ = tri.sig * lat[i] * lat[j] * vv;
-                        for ( int i = 0; i < 3; ++i )
-                            for ( int j = 0; j < 3; ++j )
-                                *set++ = tri.sig * LateralTriangle::dot( u[i], tri.v ) * lat[j];
-                    }
-                }
-}
-
-const double* grad_geometry( const tn_mesh* m )
-{
-    tn_mesh*                     mm = const_cast< tn_mesh* >( m );
-    std::lock_guard< std::mutex > lock( mm->geom_mutex );
-    if ( !mm->d_grad_geom )
-    {
-        std::vector< double > G;
-        build_grad_geometry( m, G );
-        double* p = nullptr;
-        if ( cudaMalloc( &p, G.size() * sizeof( double ) ) != cudaSuccess )
-            return nullptr;
-        if ( cudaMemcpy( p, G.data(), G.size() * sizeof( double ), cudaMemcpyHostToDevice ) != cudaSuccess )
-        {
-            cudaFree( p );
-            return nullptr;
-        }
-        mm->d_grad_geom = p;
-    }
-    return mm->d_grad_geom;
-}
 
 }  // namespace
 
@@ -412,20 +368,20 @@ int divkgrad_apply( const tn_mesh* m, const T* k, int treat, int diag, int singl
 {
     TN_CHECK_ARG( m && k && src && dst, "divkgrad_apply: null argument" );
     TN_CHECK_ARG( apply_mode == TN_APPLY_REPLACE || apply_mode == TN_APPLY_ADD, "divkgrad_apply: bad apply mode" );
-    GradParams< T > P{};
-    scalar_modes( m->N, treat, diag, P.mode_first, P.mode_inner, P.mode_last );
+    DivKGradParams< T > P{};
     if ( apply_mode == TN_APPLY_REPLACE )
         TN_CUDA_TRY( cudaMemsetAsync( dst, 0, m->ns * sizeof( T ), st ) );
-    P.N = m->N, P.n1 = m->n1, P.geom = grad_geometry( m );
-    if ( !P.geom )
-    {
-        set_error( "divkgrad_apply: allocating the lateral quadrature table failed" );
-        return TN_ERR_NOMEM;
-    }
-    P.radii = sizeof( T ) == 8 ? reinterpret_cast< const T* >( m->d_radii ) : reinterpret_cast< const T* >( m->d_radii32 );
-    P.k = k, P.src = src, P.dst = dst, P.single = single != 0;
+    P.N = m->N, P.n1 = m->n1, P.table = triangle_table< T >( m );
+    P.k = k, P.src = src, P.dst = dst, P.single = single != 0, P.treat = treat != 0;
     const long long cells = (long long) kDiamonds * m->N * m->N * m->N;
-    divkgrad_cell_kernel< T ><<< unsigned( ( cells + 127 ) / 128 ), 128, 0, st >>>( P );
+    P.cell_blocks         = unsigned( ( cells + 127 ) / 128 );
+    const unsigned edge   = P.treat ? ( boundary_items( m->N ) + 127u ) / 128u : 0u;
+    if ( diag )
+        divkgrad_diagonal_kernel< T ><<< dim3( P.cell_blocks, 4 ), 128, 0, st >>>( P );
+    else if ( single )
+        divkgrad_kernel< T, true ><<< P.cell_blocks + edge, 128, 0, st >>>( P );
+    else
+        divkgrad_kernel< T, false ><<< P.cell_blocks + edge, 128, 0, st >>>( P );
     TN_LAUNCH_CHECK();
     if ( comm_mode == TN_COMM_ADDITIVE )
         return halo_sum< T >( m, &dst, 1, st );
