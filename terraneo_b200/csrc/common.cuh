@@ -144,7 +144,6 @@ struct tn_mesh
     float*  d_triangles32 = nullptr;
 
     std::mutex      geom_mutex; // guards the tables built on first use
-    double*         d_stokes_geom = nullptr; // Divergence / Gradient, this mesh as the velocity mesh
 
     // fs/fs penalty: the orthonormalised modes are m = C (e_j x x); G = C^T C
     double penalty_gram_inv[9] = { 0 };

@@ -475,7 +475,6 @@ extern "C" int tn_mesh_destroy( tn_mesh* m )
         cudaFree( t->rad32 );
     }
     cudaFree( m->d_triangles );
-    cudaFree( m->d_stokes_geom );
     cudaFree( m->d_red_partials );
     cudaFree( m->d_red_result );
     cudaFree( m->d_red_counter );
