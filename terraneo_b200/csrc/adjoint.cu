@@ -14,11 +14,19 @@
 // does not enter.  In the interior c_w = |det J| (2 E(u):E(lambda) -
 // 2/3 div u div lambda) at the single quadrature point.
 //
-// One thread per cell, the two wedges in registers, one atomic per cell node.
+// One thread per cell (r fastest).  In the factored form of cell.cuh the scaled
+// gradient matrix at the centroid is beta_1 (x) S_1 + beta_2 (x) S_2 + v (x) Z with
+// edge differences S_i and Z = rho T - (S_1 + S_2) / 3, so a wedge needs no
+// Jacobian: about 120 multiply-adds for both fields.  The cell's node sums go out
+// by add_column.  Cells of a boundary layer with a condition are left to the first
+// blocks of the launch (one thread per lateral cell, wedge and side), which add the boundary
+// terms: with the lanes along r, every warp would otherwise carry that code for
+// one lane.  Level-6 free-slip FP64: 612 -> 132 us, FP32 276 -> 95 us.
 // Without communication the result is the derivative with respect to each
 // stored copy of k (each diamond's wedges use their own copy); with the
 // additive halo it is the derivative with respect to the unique node's value,
 // stored on all of its copies.
+#include "cell.cuh"
 #include "common.cuh"
 #include "wedge.cuh"
 
@@ -33,122 +41,169 @@ template < typename T >
 struct KGradParams
 {
     int             N, n1;
-    const double*   coords;
-    const T*        radii;
+    const double*   coords; // lateral points (unit vectors: the outward normals)
+    const T*        table;
     Ptr3< const T > u, lam;
     T*              out;
     int             bc_cmb, bc_surf;
+    unsigned        edge_blocks; // blocks of boundary cells, before those of all cells
 };
 
+// scaled gradient matrix (times 3: the weights 1/3 of the centroid, whose rounding every wedge would share, are left to
+// the one factor 1/54 at the end) of the node values s of a wedge at its centroid
 template < typename T >
-__device__ __forceinline__ void tangential( const T n[3], T v[3] )
+__device__ __forceinline__ void centroid_gradient( const Triangle< T >& G, T rho, const T ( &s )[6][3], T ( &M )[3][3] )
 {
-    const T dt = n[0] * v[0] + n[1] * v[1] + n[2] * v[2];
-    v[0] -= dt * n[0], v[1] -= dt * n[1], v[2] -= dt * n[2];
+#pragma unroll
+    for ( int c = 0; c < 3; ++c )
+    {
+        const T S1 = T( 0.5 ) * ( ( s[1][c] - s[0][c] ) + ( s[4][c] - s[3][c] ) );
+        const T S2 = T( 0.5 ) * ( ( s[2][c] - s[0][c] ) + ( s[5][c] - s[3][c] ) );
+        const T t  = ( s[3][c] - s[0][c] ) + ( s[4][c] - s[1][c] ) + ( s[5][c] - s[2][c] );
+        const T Z = T( 0.5 ) * rho * t - S1 - S2, S13 = T( 3 ) * S1, S23 = T( 3 ) * S2;
+#pragma unroll
+        for ( int a = 0; a < 3; ++a )
+            M[a][c] = G.b1[a] * S13 + G.b2[a] * S23 + G.v[a] * Z;
+    }
+}
+
+// 2 E(u) : E(l) - 2/3 div u div l of two gradient matrices
+template < typename T >
+__device__ __forceinline__ T strain_product( const T ( &A )[3][3], const T ( &B )[3][3] )
+{
+    const T tr = ( A[0][0] + A[1][1] + A[2][2] ) * ( B[0][0] + B[1][1] + B[2][2] );
+    return T( 2 ) * ( A[0][0] * B[0][0] + A[1][1] * B[1][1] + A[2][2] * B[2][2] ) +
+           ( A[0][1] + A[1][0] ) * ( B[0][1] + B[1][0] ) + ( A[0][2] + A[2][0] ) * ( B[0][2] + B[2][0] ) +
+           ( A[1][2] + A[2][1] ) * ( B[1][2] + B[2][1] ) - T( 2.0 / 3.0 ) * tr;
+}
+
+// the values of field f at the nodes of a wedge (id: wedge_columns)
+template < typename T >
+__device__ __forceinline__ void wedge_values( const Ptr3< const T >& f, const unsigned ( &id )[3], T ( &v )[6][3] )
+{
+#pragma unroll
+    for ( int n = 0; n < 6; ++n )
+#pragma unroll
+        for ( int a = 0; a < 3; ++a )
+            v[n][a] = f.p[a][id[n % 3] + n / 3];
+}
+
+// Takes the boundary condition bc out of the values v of a wedge's boundary side (top: nodes 3..5): Dirichlet values
+// are zeroed, free-slip ones projected.  b[m][.]: what was taken out, all three components or (b[m][0]) the normal one.
+template < typename T >
+__device__ __forceinline__ void split_boundary( const T ( &nn )[3][3], int bc, bool top, T ( &v )[6][3], T ( &b )[3][3] )
+{
+#pragma unroll
+    for ( int m = 0; m < 3; ++m )
+    {
+        T s[3], t[3];
+#pragma unroll
+        for ( int a = 0; a < 3; ++a )
+            s[a] = top ? v[3 + m][a] : v[m][a];
+        const T un = dot3( nn[m], s );
+#pragma unroll
+        for ( int a = 0; a < 3; ++a )
+        {
+            t[a]    = bc == TN_BC_DIRICHLET ? T( 0 ) : s[a] - un * nn[m][a];
+            b[m][a] = bc == TN_BC_DIRICHLET ? s[a] : un;
+            if ( top )
+                v[3 + m][a] = t[a];
+            else
+                v[m][a] = t[a];
+        }
+    }
+}
+
+// Cells of the layers with a boundary condition (the first edge_blocks blocks): one thread per lateral cell, wedge and
+// side.  A cell has a condition on one side (N > 1).
+template < typename T >
+__device__ __forceinline__ void kgrad_boundary( const KGradParams< T >& P )
+{
+    int  d, x, y, r, w;
+    bool top;
+    if ( !boundary_item( blockIdx.x * blockDim.x + threadIdx.x, P.N, d, x, y, r, w, top ) )
+        return;
+    const int bc = top ? P.bc_surf : P.bc_cmb;
+    if ( bc == 0 )
+        return;
+    const Triangle< T > G( P.table, P.N, d, x, y, w );
+    const T             h = layer_h( P.table, P.N, r ), rho = layer_q( P.table, P.N, r ) + T( 1 );
+    unsigned            node[4], id[3];
+    T                   nn[3][3], v[6][3], A[3][3], B[3][3], ub[3][3], lb[3][3], bnd = T( 0 );
+    cell_nodes( P.n1, d, x, y, r, node );
+    wedge_columns( node, w, id );
+#pragma unroll
+    for ( int m = 0; m < 3; ++m )
+#pragma unroll
+        for ( int a = 0; a < 3; ++a )
+            nn[m][a] = T( P.coords[size_t( ( id[m] - unsigned( r ) ) / unsigned( P.n1 ) ) * 3 + a] );
+    wedge_values( P.u, id, v );
+    split_boundary( nn, bc, top, v, ub );
+    centroid_gradient( G, rho, v, A );
+    wedge_values( P.lam, id, v );
+    split_boundary( nn, bc, top, v, lb );
+    centroid_gradient( G, rho, v, B );
+#pragma unroll
+    for ( int m = 0; m < 3; ++m )
+    {
+        T g[3];
+        scaled_gradient( G, m, top ? T( 1 ) : T( -1 ), T( 1.0 / 3.0 ), T( 1.0 / 3.0 ), T( 0 ), rho, g );
+        const T gg = dot3( g, g );
+        if ( bc == TN_BC_DIRICHLET )
+        {
+#pragma unroll
+            for ( int a = 0; a < 3; ++a )
+                bnd += lb[m][a] * ub[m][a] * ( gg + g[a] * g[a] * T( 1.0 / 3.0 ) );
+        }
+        else
+        {
+            const T ng = dot3( nn[m], g );
+            bnd += ( gg + ng * ng * T( 1.0 / 3.0 ) ) * ub[m][0] * lb[m][0];
+        }
+    }
+    const T cw = h * fabs( G.iD ) * ( strain_product( A, B ) + T( 9 ) * bnd ) * T( 1.0 / 54.0 );
+#pragma unroll
+    for ( int n = 0; n < 6; ++n )
+        atomicAdd( P.out + id[n % 3] + n / 3, cw );
 }
 
 template < typename T >
-__global__ void __launch_bounds__( 128 ) kgrad_cell_kernel( KGradParams< T > P )
+__global__ void __launch_bounds__( 128, 4 ) kgrad_kernel( KGradParams< T > P )
 {
-    const int       N = P.N, n1 = P.n1;
-    const long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x;
-    if ( t >= (long long) kDiamonds * N * N * N )
+    if ( blockIdx.x < P.edge_blocks )
+    {
+        kgrad_boundary( P );
         return;
-    const int r = int( t % N );
-    const int y = int( ( t / N ) % N );
-    const int x = int( ( t / ( (long long) N * N ) ) % N );
-    const int d = int( t / ( (long long) N * N * N ) );
-
-    const bool at_cmb = r == 0, at_surf = r == N - 1;
-    const bool cmb_dir = at_cmb && P.bc_cmb == TN_BC_DIRICHLET, surf_dir = at_surf && P.bc_surf == TN_BC_DIRICHLET;
-    const bool cmb_fs = at_cmb && P.bc_cmb == TN_BC_FREESLIP, surf_fs = at_surf && P.bc_surf == TN_BC_FREESLIP;
-    const T    r0 = P.radii[d * n1 + r], r1 = P.radii[d * n1 + r + 1];
-    const T    third = T( 1.0 / 3.0 );
-
-    T acc[2][2][2];
-    for ( int i = 0; i < 8; ++i )
-        ( &acc[0][0][0] )[i] = T( 0 );
-
+    }
+    const int  N = P.N, n1 = P.n1;
+    int        d, x, y, r;
+    const bool in = cell_of( ( blockIdx.x - P.edge_blocks ) * (long long) blockDim.x + threadIdx.x, N, d, x, y, r );
+    const T    h = layer_h( P.table, N, r ), rho = layer_q( P.table, N, r ) + T( 1 );
+    unsigned   node[4];
+    T          cw[2];
+    cell_nodes( n1, d, x, y, r, node );
+#pragma unroll
     for ( int w = 0; w < 2; ++w )
     {
-        T p[3][3], up[6][3], lp[6][3], nrm[6][3];
-        T bnd = T( 0 ); // boundary diagonal terms of the wedge (before |det J|)
-        bool dir[6], fs[6];
-        for ( int n = 0; n < 6; ++n )
-        {
-            const size_t  lat = lat_index( n1, d, x + kWedgeNode[w][n][0], y + kWedgeNode[w][n][1] );
-            const double* c   = P.coords + lat * 3;
-            if ( n < 3 )
-                for ( int a = 0; a < 3; ++a )
-                    p[n][a] = T( c[a] );
-            const T cc[3] = { T( c[0] ), T( c[1] ), T( c[2] ) };
-            const T mm    = sqrt( cc[0] * cc[0] + cc[1] * cc[1] + cc[2] * cc[2] );
-            for ( int a = 0; a < 3; ++a )
-                nrm[n][a] = cc[a] / mm;
-            const size_t i = lat * n1 + r + kWedgeNode[w][n][2];
-            for ( int a = 0; a < 3; ++a )
-            {
-                up[n][a] = P.u.p[a][i];
-                lp[n][a] = P.lam.p[a][i];
-            }
-            dir[n] = ( cmb_dir && n < 3 ) || ( surf_dir && n >= 3 );
-            fs[n]  = ( cmb_fs && n < 3 ) || ( surf_fs && n >= 3 );
-        }
-        T       IT[3][3];
-        const T det = wedge_jacobian_it( p[0], p[1], p[2], r0, r1, third, third, T( 0 ), IT );
-        T       g[6][3];
-        for ( int n = 0; n < 6; ++n )
-        {
-            T gr[3];
-            grad_shape_ref( n, third, third, T( 0 ), gr );
-            for ( int a = 0; a < 3; ++a )
-                g[n][a] = IT[a][0] * gr[0] + IT[a][1] * gr[1] + IT[a][2] * gr[2];
-        }
-        for ( int n = 0; n < 6; ++n )
-        {
-            const T gg = g[n][0] * g[n][0] + g[n][1] * g[n][1] + g[n][2] * g[n][2];
-            if ( dir[n] )
-            {
-                for ( int a = 0; a < 3; ++a )
-                    bnd += lp[n][a] * up[n][a] * ( gg + g[n][a] * g[n][a] * third );
-            }
-            else if ( fs[n] )
-            {
-                const T ng = nrm[n][0] * g[n][0] + nrm[n][1] * g[n][1] + nrm[n][2] * g[n][2];
-                const T un = nrm[n][0] * up[n][0] + nrm[n][1] * up[n][1] + nrm[n][2] * up[n][2];
-                const T ln = nrm[n][0] * lp[n][0] + nrm[n][1] * lp[n][1] + nrm[n][2] * lp[n][2];
-                bnd += ( gg + ng * ng * third ) * un * ln;
-                tangential( nrm[n], up[n] );
-                tangential( nrm[n], lp[n] );
-            }
-        }
-        // interior form on the coupled (non-Dirichlet) nodes
-        T Gu[3][3] = { { 0 } }, Gl[3][3] = { { 0 } };
-        for ( int n = 0; n < 6; ++n )
-        {
-            if ( dir[n] )
-                continue;
-            for ( int a = 0; a < 3; ++a )
-                for ( int b = 0; b < 3; ++b )
-                {
-                    Gu[a][b] += g[n][a] * up[n][b];
-                    Gl[a][b] += g[n][a] * lp[n][b];
-                }
-        }
-        T ee = T( 0 );
-        for ( int a = 0; a < 3; ++a )
-            for ( int b = 0; b < 3; ++b )
-                ee += ( Gu[a][b] + Gu[b][a] ) * ( Gl[a][b] + Gl[b][a] );
-        const T divu = Gu[0][0] + Gu[1][1] + Gu[2][2], divl = Gl[0][0] + Gl[1][1] + Gl[2][2];
-        // 2 E(u):E(l) = (1/2) sum (Gu + Gu^T)(Gl + Gl^T)
-        const T cw = fabs( det ) * ( T( 0.5 ) * ee - T( 2.0 / 3.0 ) * divu * divl + bnd ) / T( 6 );
-        for ( int n = 0; n < 6; ++n )
-            acc[kWedgeNode[w][n][0]][kWedgeNode[w][n][1]][kWedgeNode[w][n][2]] += cw;
+        const Triangle< T > G( P.table, N, d, x, y, w );
+        T                   v[6][3], A[3][3], B[3][3];
+        unsigned            id[3];
+        wedge_columns( node, w, id );
+        wedge_values( P.u, id, v );
+        centroid_gradient( G, rho, v, A );
+        wedge_values( P.lam, id, v );
+        centroid_gradient( G, rho, v, B );
+        cw[w] = h * fabs( G.iD ) * strain_product( A, B ) * T( 1.0 / 54.0 );
     }
-    for ( int dx = 0; dx < 2; ++dx )
-        for ( int dy = 0; dy < 2; ++dy )
-            for ( int dr = 0; dr < 2; ++dr )
-                atomicAdd( P.out + lat_index( n1, d, x + dx, y + dy ) * n1 + r + dr, acc[dx][dy][dr] );
+    if ( ( r == 0 && P.bc_cmb ) || ( r == N - 1 && P.bc_surf ) ) // a boundary cell: kgrad_boundary's
+        cw[0] = cw[1] = T( 0 );
+    T* const out[1] = { P.out };
+#pragma unroll
+    for ( int i = 0; i < 4; ++i )
+    {
+        const T v[1] = { i == 0 ? cw[0] : ( i == 3 ? cw[1] : cw[0] + cw[1] ) };
+        add_column< T, 1 >( out, node[i], r, N, in, true, true, v, v );
+    }
 }
 
 }  // namespace
@@ -167,10 +222,11 @@ int epsdivdiv_kgrad( const tn_mesh* m, int bc_cmb, int bc_surf, int comm_mode, c
         P.lam.p[c] = lam[c];
     }
     P.N = m->N, P.n1 = m->n1, P.coords = m->d_coords, P.out = out, P.bc_cmb = bc_cmb, P.bc_surf = bc_surf;
-    P.radii = sizeof( T ) == 8 ? reinterpret_cast< const T* >( m->d_radii ) : reinterpret_cast< const T* >( m->d_radii32 );
+    P.table = triangle_table< T >( m );
     TN_CUDA_TRY( cudaMemsetAsync( out, 0, m->ns * sizeof( T ), st ) );
     const long long cells = (long long) kDiamonds * m->N * m->N * m->N;
-    kgrad_cell_kernel< T ><<< unsigned( ( cells + 127 ) / 128 ), 128, 0, st >>>( P );
+    P.edge_blocks = bc_cmb || bc_surf ? ( boundary_items( m->N ) + 127u ) / 128u : 0u;
+    kgrad_kernel< T ><<< P.edge_blocks + unsigned( ( cells + 127 ) / 128 ), 128, 0, st >>>( P );
     TN_LAUNCH_CHECK();
     if ( comm_mode != TN_COMM_ADDITIVE )
         return TN_OK;
