@@ -8,11 +8,23 @@
 // FV ghost map); radial ghosts hold what the boundary treatment writes.
 //
 // Every kernel runs one thread per interior cell, r fastest.  The cell
-// geometry (face fluxes beta, face vectors S, volume M) is recomputed from the
-// wedge map and the Q1 velocity in FP64 in the dt and predictor kernels, with
-// the reference's face and volume quadrature sums evaluated in closed form
-// (fv_geometry).  The antidiffusive fluxes are stored as six planes (SoA),
-// F[n * nf + i] for neighbour n of cell i.
+// geometry (face fluxes beta, face vectors S, volume M) is formed from the
+// mesh's triangle vectors (cell.cuh) and the Q1 velocity in FP64 in the dt and
+// predictor kernels, with the reference's face and volume quadrature sums
+// evaluated in closed form (fv_geometry).
+//
+// The antidiffusive flux of cell i towards neighbour j is F_ij = dt / M_i
+// |beta_ij| / 2 (T_i - T_j): apart from M_i it is the same for both sides of a
+// face with opposite signs, so one value per face is stored,
+//     g = |beta| / 2 (T_i - T_j) of cell i's face towards its lower neighbour j,
+// three planes instead of six (48 bytes per cell less over the step's one write
+// and two reads; those and T_L, R+ and R- are what bounds the step).  A cell takes
+// its upper faces from its upper neighbours' entries; the last cell in a direction
+// stores its own upper face in the ghost cell there.  Level 7 (20,971,520 cells):
+// step 2.09 -> 1.39 ms, stable dt 0.81 -> 0.53 ms.
+#include <algorithm>
+
+#include "cell.cuh"
 #include "common.cuh"
 #include "wedge.cuh"
 
@@ -33,17 +45,12 @@ __device__ __forceinline__ size_t fv_index( int n2, int d, int x, int y, int r )
 struct FvGeom
 {
     int                  N;
-    const double*        coords;
+    const double*        table; // triangles (cell.cuh)
     const double*        radii;
     Ptr3< const double > cen; // FV cell centres with ghosts
     Ptr3< const double > vel; // Q1 velocity (stored nodes)
     const uint8_t*       orient; // face orientation bits per cell (nullptr: the centre test)
 };
-
-__device__ __forceinline__ void cross3( const double a[3], const double b[3], double c[3] )
-{
-    c[0] = a[1] * b[2] - a[2] * b[1], c[1] = a[2] * b[0] - a[0] * b[2], c[2] = a[0] * b[1] - a[1] * b[0];
-}
 
 // GeometryHelper::compute_geometry (geometry_helper.hpp:180-363) in closed form.
 //
@@ -65,14 +72,16 @@ __device__ __forceinline__ void cross3( const double a[3], const double b[3], do
 //     radial shape functions; the quad eta = 0 alike with a in place of b and
 //     nodes 1, 4 in place of 2, 5;
 //   * det J = r(zeta)^2 h (a x b) . p0, so M = sum_w h |(a x b) . p0|
-//     (r(-g)^2 + r(g)^2) / 2.
+//     (r(-g)^2 + r(g)^2) / 2: a lateral factor times a radial one, whose inverses
+//     are tabulated (iM = 1 / M, fv_inverse_volume).
 // These are the same sums (exact algebra, different rounding: ~1e-16
-// relative), about 150 FP64 operations per cell instead of ~3,000.  Every face
-// is then oriented from this cell towards the neighbour's centre.
+// relative), about 120 FP64 operations per cell instead of ~3,000, with b x p0,
+// a x p0 = -(p0 x a), a x b and 1 / ((a x b) . p0) from the triangle table.  Every
+// face is then oriented from this cell towards the neighbour's centre.
 // WITH_VELOCITY: the face fluxes beta (false: geometry only); WITH_S: the face vectors S, needed by the
 // orientation test and the diffusion term only (with the orientation bits and no diffusivity they are dead).
 template < bool WITH_VELOCITY = true, bool WITH_S = true >
-__device__ void fv_geometry( const FvGeom& G, int d, int x, int y, int r, double beta[6], double& Mii, double S[6][3],
+__device__ void fv_geometry( const FvGeom& G, int d, int x, int y, int r, double beta[6], double& iM, double S[6][3],
                              uint8_t* flips = nullptr )
 {
     const int    N = G.N, n1 = N + 1, n2 = N + 2;
@@ -88,31 +97,22 @@ __device__ void fv_geometry( const FvGeom& G, int d, int x, int y, int r, double
         beta[n] = 0.0;
         S[n][0] = S[n][1] = S[n][2] = 0.0;
     }
-    Mii = 0.0;
+    unsigned node[4];
+    cell_nodes( n1, d, x - 1, y - 1, r - 1, node );
 #pragma unroll
     for ( int w = 0; w < 2; ++w )
     {
-        double p[3][3], u[6][3];
+        const Triangle< double > t( G.table, N, d, x - 1, y - 1, w );
+        double                   u[6][3];
 #pragma unroll
         for ( int i = 0; i < 6; ++i )
         {
-            const size_t lat = lat_index( n1, d, x - 1 + kWedgeNode[w][i][0], y - 1 + kWedgeNode[w][i][1] );
-            if ( i < 3 )
-#pragma unroll
-                for ( int c = 0; c < 3; ++c )
-                    p[i][c] = G.coords[lat * 3 + c];
-            const size_t id = lat * n1 + r - 1 + kWedgeNode[w][i][2];
+            const unsigned id = node[wedge_node( w, i, 0 ) + 2 * wedge_node( w, i, 1 )] + i / 3;
 #pragma unroll
             for ( int c = 0; c < 3; ++c )
                 u[i][c] = WITH_VELOCITY ? G.vel.p[c][id] : 0.0;
         }
-        double va[3], vb[3], ab[3], bp[3], ap[3];
-#pragma unroll
-        for ( int c = 0; c < 3; ++c )
-            va[c] = p[1][c] - p[0][c], vb[c] = p[2][c] - p[0][c];
-        cross3( va, vb, ab );
-        cross3( vb, p[0], bp );
-        cross3( va, p[0], ap );
+        const double *ab = t.v, *bp = t.b1, ap[3] = { -t.b2[0], -t.b2[1], -t.b2[2] };
         const int nx = w == 0 ? 0 : 1, ny = w == 0 ? 2 : 3; // the wedge's xi = 0 and eta = 0 faces
         double    bx = 0.0, by = 0.0, bl = 0.0, bt = 0.0;
 #pragma unroll
@@ -134,9 +134,8 @@ __device__ void fv_geometry( const FvGeom& G, int d, int x, int y, int r, double
         beta[ny] += h * by;
         beta[4] += r1s / 6.0 * bl;
         beta[5] += r2s / 6.0 * bt;
-        const double D = ab[0] * p[0][0] + ab[1] * p[0][1] + ab[2] * p[0][2];
-        Mii += 0.5 * h * fabs( D ) * ( rm * rm + rp * rp );
     }
+    iM = fv_inverse_volume( G.table, N, d, x - 1, y - 1, r - 1 );
     // orient every face from this cell towards the neighbour's centre: from the mesh's orientation bits (the
     // same test, made once per mesh), else the test itself
     const size_t ci   = fv_index( n2, d, x, y, r );
@@ -173,14 +172,9 @@ __device__ void fv_geometry( const FvGeom& G, int d, int x, int y, int r, double
 
 __device__ __forceinline__ bool cell_of_thread( int N, int& d, int& x, int& y, int& r )
 {
-    const long long t = blockIdx.x * (long long) blockDim.x + threadIdx.x;
-    if ( t >= (long long) kDiamonds * N * N * N )
-        return false;
-    r = int( t % N ) + 1;
-    y = int( ( t / N ) % N ) + 1;
-    x = int( ( t / ( (long long) N * N ) ) % N ) + 1;
-    d = int( t / ( (long long) N * N * N ) );
-    return true;
+    const bool in = cell_of( blockIdx.x * (long long) blockDim.x + threadIdx.x, N, d, x, y, r );
+    ++x, ++y, ++r;
+    return in;
 }
 
 // compute_cell_centers (fv/hex/helpers.hpp:101-150)
@@ -221,8 +215,9 @@ __global__ void __launch_bounds__( kFvThreads ) cell_centers_kernel( int N, cons
 }
 
 // lateral ghost layer: thread per (ghost cell, r)
-__global__ void fv_ghost_kernel( int N, const int* __restrict__ map, double* __restrict__ f )
+__global__ void fv_ghost_kernel( int N, const int* __restrict__ map, Ptr3< double > fields )
 {
+    double* f = fields.at( blockIdx.y );
     const long long t     = blockIdx.x * (long long) blockDim.x + threadIdx.x;
     const long long total = (long long) kDiamonds * 4 * N * N;
     if ( t >= total )
@@ -247,21 +242,28 @@ __global__ void __launch_bounds__( kFvThreads ) orient_kernel( FvGeom G, uint8_t
     int d, x, y, r;
     if ( !cell_of_thread( G.N, d, x, y, r ) )
         return;
-    double beta[6], Mii, S[6][3];
-    fv_geometry< false >( G, d, x, y, r, beta, Mii, S, bits + fv_index( G.N + 2, d, x, y, r ) );
+    double beta[6], iM, S[6][3];
+    fv_geometry< false >( G, d, x, y, r, beta, iM, S, bits + fv_index( G.N + 2, d, x, y, r ) );
 }
 
+// Blocks take the cells in turn and one atomic per block closes the minimum: one per warp on the single result cost
+// as much as the geometry (level 7: 655,360 of them).
 template < bool DIFFUSION >
-__global__ void __launch_bounds__( kFvThreads ) dt_kernel( FvGeom G, double kappa, unsigned long long* out )
+__global__ void __launch_bounds__( kFvThreads, 4 ) dt_kernel( FvGeom G, double kappa, unsigned long long* out )
 {
-    int    d, x, y, r;
-    double dtc = 1e300;
-    if ( cell_of_thread( G.N, d, x, y, r ) )
+    __shared__ double sh[kFvThreads / 32];
+    const long long   cells = (long long) kDiamonds * G.N * G.N * G.N;
+    const int         n2    = G.N + 2;
+    double            dtc   = 1e300;
+    for ( long long t = blockIdx.x * (long long) kFvThreads + threadIdx.x; t < cells; t += (long long) gridDim.x * kFvThreads )
     {
-        const int n2 = G.N + 2;
-        double    beta[6], Mii, S[6][3], lambda = 0.0;
-        fv_geometry< true, DIFFUSION >( G, d, x, y, r, beta, Mii, S );
+        int    d, x, y, r;
+        double beta[6], iM, S[6][3], lambda = 0.0;
+        cell_of( t, G.N, d, x, y, r );
+        ++x, ++y, ++r;
+        fv_geometry< true, DIFFUSION >( G, d, x, y, r, beta, iM, S );
         const size_t ci = fv_index( n2, d, x, y, r );
+#pragma unroll
         for ( int n = 0; n < 6; ++n )
         {
             if ( beta[n] < 0 )
@@ -279,30 +281,38 @@ __global__ void __launch_bounds__( kFvThreads ) dt_kernel( FvGeom G, double kapp
                     lambda += kappa * ss / den;
             }
         }
-        dtc = lambda > 0 ? Mii / lambda : 1e30;
+        dtc = fmin( dtc, lambda > 0 ? 1.0 / ( iM * lambda ) : 1e30 );
     }
     for ( int off = 16; off > 0; off >>= 1 )
         dtc = fmin( dtc, __shfl_down_sync( 0xffffffffu, dtc, off ) );
     if ( ( threadIdx.x & 31 ) == 0 )
+        sh[threadIdx.x >> 5] = dtc;
+    __syncthreads();
+    if ( threadIdx.x == 0 )
+    {
+        for ( int w = 1; w < kFvThreads / 32; ++w )
+            dtc = fmin( dtc, sh[w] );
         atomicMin( out, (unsigned long long) __double_as_longlong( dtc ) );
+    }
 }
 
 // FCTPredictorKernel (fct_advection_diffusion.hpp:262-376); DIFFUSION: kappa != 0
 template < bool DIFFUSION >
-__global__ void __launch_bounds__( kFvThreads )
-    predictor_kernel( FvGeom G, const double* __restrict__ T, double* __restrict__ TL, double* __restrict__ F, double dt,
+__global__ void __launch_bounds__( kFvThreads, DIFFUSION ? 4 : 6 )
+    predictor_kernel( FvGeom G, const double* __restrict__ T, double* __restrict__ TL, double* __restrict__ g, double dt,
                       double kappa, const double* __restrict__ src, int subtract_divergence )
 {
     int d, x, y, r;
     if ( !cell_of_thread( G.N, d, x, y, r ) )
         return;
     const int n2 = G.N + 2;
-    double    beta[6], Mii, S[6][3];
-    fv_geometry< true, DIFFUSION >( G, d, x, y, r, beta, Mii, S );
+    double    beta[6], iM, S[6][3];
+    fv_geometry< true, DIFFUSION >( G, d, x, y, r, beta, iM, S );
     const size_t i  = fv_index( n2, d, x, y, r );
-    const size_t nf = size_t( kDiamonds ) * n2 * n2 * n2; // F holds 6 planes of nf (SoA)
+    const size_t nf = size_t( kDiamonds ) * n2 * n2 * n2; // g holds 3 planes of nf (SoA)
     const double Ti = T[i];
     double       lo_diag = 0.0, lo_update = 0.0, bsum = 0.0;
+#pragma unroll
     for ( int n = 0; n < 6; ++n )
     {
         const size_t j  = fv_index( n2, d, x + kFvOff[n][0], y + kFvOff[n][1], r + kFvOff[n][2] );
@@ -324,11 +334,15 @@ __global__ void __launch_bounds__( kFvThreads )
             lo_diag += dc;
             lo_update -= dc * Tj;
         }
-        F[n * nf + i] = ( dt / Mii ) * ( fabs( beta[n] ) / 2.0 ) * ( Ti - Tj );
+        // face 2a towards the lower neighbour in direction a; the last cell's upper face goes to the ghost cell
+        if ( n % 2 == 0 )
+            g[( n / 2 ) * nf + i] = fabs( beta[n] ) * 0.5 * ( Ti - Tj );
+        else if ( ( n == 1 ? x : ( n == 3 ? y : r ) ) == G.N )
+            g[( n / 2 ) * nf + j] = fabs( beta[n] ) * 0.5 * ( Tj - Ti );
     }
     if ( subtract_divergence )
         lo_diag -= bsum;
-    double tl = Ti - ( dt / Mii ) * ( lo_diag * Ti + lo_update );
+    double tl = Ti - ( dt * iM ) * ( lo_diag * Ti + lo_update );
     if ( src )
         tl += dt * src[i];
     TL[i] = tl;
@@ -348,26 +362,38 @@ __global__ void dirichlet_kernel( int N, double* __restrict__ T, double t_cmb, d
         T[fv_index( n2, d, x, y, N )] = T[fv_index( n2, d, x, y, N + 1 )] = t_surf;
 }
 
+// the six antidiffusive fluxes of cell i (dt / M_i times its faces' g)
+__device__ __forceinline__ void antidiffusive( const double* __restrict__ g, size_t nf, int n2, size_t i, double scale, double f[6] )
+{
+    const size_t step[3] = { size_t( n2 ) * n2, size_t( n2 ), 1 };
+#pragma unroll
+    for ( int a = 0; a < 3; ++a )
+    {
+        f[2 * a]     = scale * g[a * nf + i];
+        f[2 * a + 1] = -scale * g[a * nf + i + step[a]];
+    }
+}
+
 // FCTLimiterKernel (fct_advection_diffusion.hpp:486-531)
-__global__ void __launch_bounds__( kFvThreads ) limiter_kernel( int N, const double* __restrict__ TL,
-                                                                const double* __restrict__ F, double* __restrict__ Rp,
-                                                                double* __restrict__ Rm )
+__global__ void __launch_bounds__( kFvThreads )
+    limiter_kernel( FvGeom G, const double* __restrict__ TL, const double* __restrict__ g, double dt, double* __restrict__ Rp,
+                    double* __restrict__ Rm )
 {
     int d, x, y, r;
-    if ( !cell_of_thread( N, d, x, y, r ) )
+    if ( !cell_of_thread( G.N, d, x, y, r ) )
         return;
-    const int    n2 = N + 2;
+    const int    n2 = G.N + 2;
     const size_t i  = fv_index( n2, d, x, y, r );
-    const size_t nf = size_t( kDiamonds ) * n2 * n2 * n2;
     const double ti = TL[i];
-    double       Pp = 0.0, Pm = 0.0, tmax = ti, tmin = ti;
+    double       f[6], Pp = 0.0, Pm = 0.0, tmax = ti, tmin = ti;
+    antidiffusive( g, size_t( kDiamonds ) * n2 * n2 * n2, n2, i, dt * fv_inverse_volume( G.table, G.N, d, x - 1, y - 1, r - 1 ), f );
+#pragma unroll
     for ( int n = 0; n < 6; ++n )
     {
-        const double f = F[n * nf + i];
-        if ( f > 0 )
-            Pp += f;
+        if ( f[n] > 0 )
+            Pp += f[n];
         else
-            Pm += f;
+            Pm += f[n];
         const double tj = TL[fv_index( n2, d, x + kFvOff[n][0], y + kFvOff[n][1], r + kFvOff[n][2] )];
         tmax            = fmax( tmax, tj );
         tmin            = fmin( tmin, tj );
@@ -378,24 +404,50 @@ __global__ void __launch_bounds__( kFvThreads ) limiter_kernel( int N, const dou
 
 // FCTCorrectionKernel (fct_advection_diffusion.hpp:605-650)
 __global__ void __launch_bounds__( kFvThreads )
-    correction_kernel( int N, const double* __restrict__ TL, const double* __restrict__ F,
+    correction_kernel( FvGeom G, const double* __restrict__ TL, const double* __restrict__ g, double dt,
                        const double* __restrict__ Rp, const double* __restrict__ Rm, double* __restrict__ T )
 {
     int d, x, y, r;
-    if ( !cell_of_thread( N, d, x, y, r ) )
+    if ( !cell_of_thread( G.N, d, x, y, r ) )
         return;
-    const int    n2 = N + 2;
+    const int    n2 = G.N + 2;
     const size_t i  = fv_index( n2, d, x, y, r );
-    const size_t nf = size_t( kDiamonds ) * n2 * n2 * n2;
-    double       corr = 0.0;
+    const double rp = Rp[i], rm = Rm[i];
+    double       f[6], corr = 0.0;
+    antidiffusive( g, size_t( kDiamonds ) * n2 * n2 * n2, n2, i, dt * fv_inverse_volume( G.table, G.N, d, x - 1, y - 1, r - 1 ), f );
+#pragma unroll
     for ( int n = 0; n < 6; ++n )
     {
         const size_t j  = fv_index( n2, d, x + kFvOff[n][0], y + kFvOff[n][1], r + kFvOff[n][2] );
-        const double f  = F[n * nf + i];
-        const double al = f > 0 ? fmin( Rp[i], Rm[j] ) : fmin( Rm[i], Rp[j] );
-        corr += al * f;
+        const double al = f[n] > 0 ? fmin( rp, Rm[j] ) : fmin( rm, Rp[j] );
+        corr += al * f[n];
     }
     T[i] = TL[i] + corr;
+}
+
+// Zeroes the ghost cells (all those outside 1..N in some direction) of nf fields: the first and last cell of every
+// column, one thread per column, and whole ghost columns, one thread per cell of them (blocks after the first
+// col_blocks).
+__global__ void __launch_bounds__( 256 ) fv_zero_ghost_kernel( int N, Ptr3< double > f, int nf, unsigned col_blocks )
+{
+    const unsigned n2 = unsigned( N ) + 2, cols = unsigned( kDiamonds ) * n2 * n2, ring = 4 * ( n2 - 1 );
+    if ( blockIdx.x < col_blocks )
+    {
+        const unsigned c = blockIdx.x * blockDim.x + threadIdx.x;
+        if ( c < cols )
+            for ( int k = 0; k < nf; ++k )
+                f.at( k )[size_t( c ) * n2] = f.at( k )[size_t( c ) * n2 + n2 - 1] = 0.0;
+        return;
+    }
+    const unsigned t = ( blockIdx.x - col_blocks ) * blockDim.x + threadIdx.x, e = t / n2, r = t % n2;
+    if ( e >= unsigned( kDiamonds ) * ring )
+        return;
+    // column e % ring around the diamond: sides x = 0, y = n2 - 1, x = n2 - 1, y = 0 of n2 - 1 columns each
+    const unsigned d = e / ring, s = e % ring / ( n2 - 1 ), i = e % ( n2 - 1 );
+    const unsigned x = s == 0 ? 0u : ( s == 1 ? i : ( s == 2 ? n2 - 1 : n2 - 1 - i ) );
+    const unsigned y = s == 0 ? i : ( s == 1 ? n2 - 1 : ( s == 2 ? n2 - 1 - i : 0u ) );
+    for ( int k = 0; k < nf; ++k )
+        f.at( k )[( ( size_t( d ) * n2 + x ) * n2 + y ) * n2 + r] = 0.0;
 }
 
 size_t fv_size( const tn_mesh* m )
@@ -409,10 +461,12 @@ unsigned cell_blocks( const tn_mesh* m )
     return unsigned( ( (long long) kDiamonds * m->N * m->N * m->N + kFvThreads - 1 ) / kFvThreads );
 }
 
-int ghost_update( const tn_mesh* m, double* f, cudaStream_t st )
+// lateral ghosts of one field, or of two in one launch
+int ghost_update( const tn_mesh* m, double* f, cudaStream_t st, double* f2 = nullptr )
 {
     const long long n = (long long) kDiamonds * 4 * m->N * m->N;
-    fv_ghost_kernel<<< unsigned( ( n + 255 ) / 256 ), 256, 0, st >>>( m->N, m->d_fv_ghost, f );
+    fv_ghost_kernel<<< dim3( unsigned( ( n + 255 ) / 256 ), f2 ? 2 : 1 ), 256, 0, st >>>( m->N, m->d_fv_ghost,
+                                                                                         Ptr3< double >{ { f, f2, nullptr } } );
     TN_LAUNCH_CHECK();
     return TN_OK;
 }
@@ -420,7 +474,7 @@ int ghost_update( const tn_mesh* m, double* f, cudaStream_t st )
 // The face orientation bits of the mesh, from its own cell centres (compute_cell_centers, the centres
 // tn_fv_cell_centers_f64 gives), built on the first FCT call of the mesh: the orientation is geometry, so the
 // per-step kernels read one byte per cell instead of the six neighbours' centres.
-const uint8_t* fv_orientation( const tn_mesh* m, cudaStream_t st )
+const uint8_t* fv_orientation( const tn_mesh* m, const double* table, cudaStream_t st )
 {
     tn_mesh*                      mm = const_cast< tn_mesh* >( m );
     std::lock_guard< std::mutex > lock( mm->geom_mutex );
@@ -449,7 +503,7 @@ const uint8_t* fv_orientation( const tn_mesh* m, cudaStream_t st )
         if ( ok )
         {
             FvGeom G{};
-            G.N = m->N, G.coords = m->d_coords, G.radii = m->d_radii;
+            G.N = m->N, G.table = table, G.radii = m->d_radii;
             G.cen    = Ptr3< const double >{ { c, c + nf, c + 2 * nf } };
             G.orient = nullptr;
             orient_kernel<<< cell_blocks( m ), kFvThreads, 0, st >>>( G, b );
@@ -475,8 +529,8 @@ int make_geom( const tn_mesh* m, const double* const* vel, const double* const* 
         G.vel.p[a] = vel[a];
         G.cen.p[a] = cen[a];
     }
-    G.N = m->N, G.coords = m->d_coords, G.radii = m->d_radii;
-    G.orient = fv_orientation( m, st );
+    G.N = m->N, G.table = triangle_table< double >( m ), G.radii = m->d_radii;
+    G.orient = fv_orientation( m, G.table, st );
     if ( !G.orient )
     {
         set_error( "fct: building the face orientation of the mesh failed" );
@@ -539,12 +593,13 @@ extern "C" int tn_fct_dt_stable_f64( const tn_mesh* m, const double* const* vel,
     if ( ( rc = make_geom( m, vel, centers, G, st ) ) )
         return rc;
     unsigned long long* slot = reinterpret_cast< unsigned long long* >( m->d_red_result + 12 );
-    const double        init = 1e300;
-    TN_CUDA_TRY( cudaMemcpyAsync( slot, &init, sizeof( double ), cudaMemcpyHostToDevice, st ) );
+    // bytes 0x7f: 1.4e306, above every candidate
+    TN_CUDA_TRY( cudaMemsetAsync( slot, 0x7f, sizeof( double ), st ) );
+    const unsigned blocks = std::min( cell_blocks( m ), 148u * 16u );
     if ( diffusivity != 0.0 )
-        dt_kernel< true ><<< cell_blocks( m ), kFvThreads, 0, st >>>( G, diffusivity, slot );
+        dt_kernel< true ><<< blocks, kFvThreads, 0, st >>>( G, diffusivity, slot );
     else
-        dt_kernel< false ><<< cell_blocks( m ), kFvThreads, 0, st >>>( G, diffusivity, slot );
+        dt_kernel< false ><<< blocks, kFvThreads, 0, st >>>( G, diffusivity, slot );
     TN_LAUNCH_CHECK();
     TN_CUDA_TRY( cudaMemcpyAsync( dt_stable, slot, sizeof( double ), cudaMemcpyDeviceToHost, st ) );
     TN_CUDA_TRY( cudaStreamSynchronize( st ) );
@@ -572,17 +627,20 @@ extern "C" int tn_fct_step_f64( const tn_mesh* m, double* T, const double* const
     if ( ( rc = make_geom( m, vel, centers, G, st ) ) )
         return rc;
     const size_t nf = fv_size( m );
-    double *     TL = workspace, *F = workspace + nf, *Rp = workspace + 7 * nf, *Rm = workspace + 8 * nf;
-    TN_CUDA_TRY( cudaMemsetAsync( TL, 0, sizeof( double ) * nf, st ) );
-    TN_CUDA_TRY( cudaMemsetAsync( Rp, 0, sizeof( double ) * 2 * nf, st ) );
+    double *     TL = workspace, *g = workspace + nf, *Rp = workspace + 7 * nf, *Rm = workspace + 8 * nf;
+    // the radial ghosts enter as zeros where no boundary treatment sets them; every interior cell is written below
+    const unsigned n2 = unsigned( m->N ) + 2, col_blocks = ( unsigned( kDiamonds ) * n2 * n2 + 255u ) / 256u;
+    const unsigned ring_blocks = ( unsigned( kDiamonds ) * 4u * ( n2 - 1 ) * n2 + 255u ) / 256u;
+    fv_zero_ghost_kernel<<< col_blocks + ring_blocks, 256, 0, st >>>( m->N, Ptr3< double >{ { TL, Rp, Rm } }, 3, col_blocks );
+    TN_LAUNCH_CHECK();
     // predictor (fct_advection_diffusion.hpp:384-433) on T with fresh lateral ghosts
     if ( ( rc = ghost_update( m, T, st ) ) )
         return rc;
     if ( diffusivity != 0.0 )
-        predictor_kernel< true ><<< cell_blocks( m ), kFvThreads, 0, st >>>( G, T, TL, F, dt, diffusivity, source,
+        predictor_kernel< true ><<< cell_blocks( m ), kFvThreads, 0, st >>>( G, T, TL, g, dt, diffusivity, source,
                                                                              subtract_divergence );
     else
-        predictor_kernel< false ><<< cell_blocks( m ), kFvThreads, 0, st >>>( G, T, TL, F, dt, diffusivity, source,
+        predictor_kernel< false ><<< cell_blocks( m ), kFvThreads, 0, st >>>( G, T, TL, g, dt, diffusivity, source,
                                                                               subtract_divergence );
     TN_LAUNCH_CHECK();
     if ( bcs && ( rc = tn_fct_apply_dirichlet_f64( m, TL, bcs, s ) ) )
@@ -590,11 +648,11 @@ extern "C" int tn_fct_step_f64( const tn_mesh* m, double* T, const double* const
     // limiter (:539-566) and correction (:658-680)
     if ( ( rc = ghost_update( m, TL, st ) ) )
         return rc;
-    limiter_kernel<<< cell_blocks( m ), kFvThreads, 0, st >>>( m->N, TL, F, Rp, Rm );
+    limiter_kernel<<< cell_blocks( m ), kFvThreads, 0, st >>>( G, TL, g, dt, Rp, Rm );
     TN_LAUNCH_CHECK();
-    if ( ( rc = ghost_update( m, Rp, st ) ) || ( rc = ghost_update( m, Rm, st ) ) )
+    if ( ( rc = ghost_update( m, Rp, st, Rm ) ) )
         return rc;
-    correction_kernel<<< cell_blocks( m ), kFvThreads, 0, st >>>( m->N, TL, F, Rp, Rm, T );
+    correction_kernel<<< cell_blocks( m ), kFvThreads, 0, st >>>( G, TL, g, dt, Rp, Rm, T );
     TN_LAUNCH_CHECK();
     return TN_OK;
 }
