@@ -154,6 +154,11 @@ struct tn_mesh
     unsigned int* d_red_counter  = nullptr;
     double*       h_red_result   = nullptr; // pinned, 16 doubles
 
+    // one block of solver memory kept between solves (WorkBlock), and its size in doubles
+    std::mutex work_mutex;
+    double*    d_work = nullptr;
+    size_t     n_work = 0;
+
     // side stream for work that overlaps a kernel of the caller's stream
     // (forked from and joined back into that stream with the two events)
     cudaStream_t side_stream = nullptr;
@@ -162,4 +167,22 @@ struct tn_mesh
 
 namespace tn {
 constexpr int kRedMaxBlocks = 1184; // 148 SMs x 8
+
+// Device memory of one solve: the mesh's kept block if it is free and large enough, else a new allocation.  The block
+// goes back to the mesh when this goes out of scope (the larger one is kept, at most one per mesh, freed with it), so
+// the owner must have waited for its stream by then; a second solve on the mesh meanwhile gets its own.
+class WorkBlock
+{
+  public:
+    WorkBlock( const tn_mesh* m, size_t n );
+    ~WorkBlock();
+    WorkBlock( const WorkBlock& ) = delete;
+    WorkBlock& operator=( const WorkBlock& ) = delete;
+    double*    get() const { return p_; } // NULL: the allocation failed
+
+  private:
+    tn_mesh* m_;
+    double*  p_ = nullptr;
+    size_t   n_;
+};
 }

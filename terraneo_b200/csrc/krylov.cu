@@ -215,16 +215,41 @@ __global__ void pcg_update_kernel( Segs s, SegPtr< T > x, SegPtr< T > r, SegPtr<
     const double alpha = state[kAn] / state[kPap];
     const T      ta = T( alpha ), tm = T( -alpha );
     Neumaier     acc;
+    // kU entries per thread and step, all loads issued before the arithmetic
+    constexpr int kU     = 4;
+    const size_t  stride = size_t( gridDim.x ) * blockDim.x;
 #pragma unroll
     for ( int k = 0; k < kMaxSegs; ++k ) // compile-time segment indices (no stack copy)
         if ( k < s.n )
-        for ( size_t i = blockIdx.x * size_t( blockDim.x ) + threadIdx.x; i < s.len[k];
-              i += size_t( gridDim.x ) * blockDim.x )
         {
-            x.p[k][i]    = x.p[k][i] + ta * p.p[k][i];
-            const T ri   = r.p[k][i] + tm * ap.p[k][i];
-            r.p[k][i]    = ri;
-            acc.add( s.owned[k][i] ? double( ri ) * double( ri ) : 0.0 );
+            T* __restrict__ px             = x.p[k];
+            T* __restrict__ pr             = r.p[k];
+            const T* __restrict__ pp       = p.p[k];
+            const T* __restrict__ pa       = ap.p[k];
+            const uint8_t* __restrict__ ow = s.owned[k];
+            const size_t n                 = s.len[k];
+            for ( size_t i0 = blockIdx.x * size_t( blockDim.x ) + threadIdx.x; i0 < n; i0 += kU * stride )
+            {
+                T       xi[kU], ri[kU], pi[kU], ai[kU];
+                uint8_t oi[kU];
+#pragma unroll
+                for ( int u = 0; u < kU; ++u )
+                {
+                    const size_t i = i0 + u * stride < n ? i0 + u * stride : i0;
+                    xi[u] = px[i], ri[u] = pr[i], pi[u] = pp[i], ai[u] = pa[i], oi[u] = ow[i];
+                }
+#pragma unroll
+                for ( int u = 0; u < kU; ++u )
+                {
+                    const size_t i = i0 + u * stride;
+                    if ( i >= n )
+                        break;
+                    const T v = ri[u] + tm * ai[u];
+                    px[i]     = xi[u] + ta * pi[u];
+                    pr[i]     = v;
+                    acc.add( oi[u] ? double( v ) * double( v ) : 0.0 );
+                }
+            }
         }
     if ( block_sum_finish< 1 >( &acc, partials, counter, scratch ) && threadIdx.x == 0 )
     {

@@ -11,7 +11,7 @@
 
 #include "cell.cuh"
 #include "common.cuh"
-#include "lateral.cuh"
+#include "lateral_cg.cuh"
 #include "wedge.cuh"
 
 namespace tn {
@@ -360,6 +360,29 @@ int laplace_apply( const tn_mesh* m, int treat, int diag, int apply_mode, int co
     const T* s[1] = { src };
     T*       d[1] = { dst };
     return constant_gradient_apply< T >( m, 1, s, d, f, i, l, apply_mode, comm_mode, st, "laplace_apply" );
+}
+
+// CG on Laplace(treat_boundary) from x's values (lateral_cg.cuh)
+int laplace_cg( const tn_mesh* m, const double* b, double* x, int max_iterations, double rtol, double atol, int* iterations,
+                double* relres, cudaStream_t st )
+{
+    LateralParams< double > P{};
+    if ( !lateral_tables< LaplaceOp< double > >( m, &tn_mesh::laplace_tables, P, st ) )
+    {
+        set_error( "laplace_cg: allocating the lateral stencils failed" );
+        return TN_ERR_NOMEM;
+    }
+    scalar_modes( m->N, 1, 0, P.mode_first, P.mode_inner, P.mode_last );
+    const size_t    ns = m->ns;
+    const WorkBlock w( m, 4 * ns + lateral_cg_scratch< LaplaceOp< double > >( m, max_iterations ) );
+    if ( !w.get() )
+    {
+        set_error( "laplace_cg: allocating the work fields failed" );
+        return TN_ERR_NOMEM;
+    }
+    double* const fields[4] = { w.get(), w.get() + ns, w.get() + 2 * ns, w.get() + 3 * ns };
+    return lateral_cg< LaplaceOp< double > >( m, P, b, x, fields, w.get() + 4 * ns, max_iterations, rtol, atol, iterations, relres,
+                                              st );
 }
 
 template < typename T >

@@ -29,9 +29,8 @@
 // Measured for the level-6 FP64 Laplacian: one thread per node with the
 // stencil read for every node 58 us, four levels per thread 56 us (bound by
 // instruction issue and the latency of those reads), runs of 22 levels staged
-// by whole warps 41 us, runs of 14 staged by half-warps 29 us, and 39 us with
-// the sums on differences (128 registers, some spilled).  What is left is
-// instruction issue (44 % of the slots).
+// by whole warps 41 us, runs of 14 staged by half-warps 29 us, and 33 us with the
+// sums on differences.  What is left is instruction issue (44 % of the slots).
 //
 // Columns on the edge of a diamond have copies in other diamonds.  With
 // additive communication their sums run over the columns of all copies (each
@@ -46,6 +45,7 @@
 #include <atomic>
 
 #include "common.cuh"
+#include "reduce.cuh"
 #include "wedge.cuh"
 
 namespace tn {
@@ -96,6 +96,19 @@ struct LateralParams
     int             mode_first, mode_inner, mode_last; // coupling of the layers, kNeu .. kDiag
 };
 
+// What a CG step adds to the apply (lateral_cg.cuh): the operand is the new direction p = r + beta p_old, formed
+// while it is read and written to p_new, and <p, A p> is summed over the owned nodes.
+struct LateralCG
+{
+    bool          live; // false: the stopping rule has fired, nothing is written
+    const double* r;
+    const double* p_old;
+    double*       p_new;
+    double*       state; // tn_pcg_* layout
+    double*       partials;
+    unsigned int* counter;
+};
+
 // a column's sums at one level: of the first S stencils, of the other D on the level's own values (used by the layers
 // that do not couple their two levels), and the products of all K self entries
 template < typename OP, typename T >
@@ -119,8 +132,9 @@ __device__ __forceinline__ void lateral_layer( int mode, const T ( &rad )[OP::R]
     }
 }
 
-template < typename OP, typename T >
-__device__ __forceinline__ void lateral_tile( const LateralParams< T >& P, unsigned block, T* smem )
+template < typename OP, bool CG, typename T >
+__device__ __forceinline__ void lateral_tile( const LateralParams< T >& P, const LateralCG& cg, T beta, unsigned block, T* smem,
+                                              Neumaier& dot )
 {
     constexpr int K = OP::K, R = OP::R;
     const int     n1 = P.n1, tid = int( threadIdx.x ), lane = tid & 31, warp = tid >> 5;
@@ -143,10 +157,21 @@ __device__ __forceinline__ void lateral_tile( const LateralParams< T >& P, unsig
         {
             const T* g = src + size_t( x ) * n1 * n1 + r;
             T*       c = in + x * ( kTileY + 2 ) * kStride + hl;
+            if constexpr ( CG )
+            {
+                const T* q = cg.r + ( g - P.src.p[0] );
 #pragma unroll
-            for ( int y = 0; y < kTileY + 2; ++y, g += n1 )
-                if ( y < ymax )
-                    __pipeline_memcpy_async( c + y * kStride, g, sizeof( T ) );
+                for ( int y = 0; y < kTileY + 2; ++y )
+                    if ( y < ymax )
+                        c[y * kStride] = q[size_t( y ) * n1] + beta * g[size_t( y ) * n1];
+            }
+            else
+            {
+#pragma unroll
+                for ( int y = 0; y < kTileY + 2; ++y, g += n1 )
+                    if ( y < ymax )
+                        __pipeline_memcpy_async( c + y * kStride, g, sizeof( T ) );
+            }
         }
     }
     for ( int i = tid; i < R * ( P.run + 1 ); i += kLateralThreads )
@@ -170,12 +195,10 @@ __device__ __forceinline__ void lateral_tile( const LateralParams< T >& P, unsig
     {
         const T* u = in + ( ( tx + 1 ) * ( kTileY + 2 ) + ty + 1 ) * kStride - ( ra - 1 ); // u[r] = level r
         T*       o = out + tid * kStride - ra;
-        T        high = T( 0 ), vb[kStencil];
+        T                  high = T( 0 );
         LevelSums< OP, T > b{};
-#pragma unroll
-        for ( int i = 0; i < kStencil; ++i )
-            vb[i] = T( 0 );
-        // sums of level l, which close the layer l - 1 below it
+        // sums of level l, which close the layer l - 1 below it (the level below is read again for the difference:
+        // held in registers it made them spill, 39 instead of 33 us)
         int below = kNeu;
         for ( int l = max( ra - 1, 0 ); l <= min( rb, P.N ); ++l )
         {
@@ -199,7 +222,7 @@ __device__ __forceinline__ void lateral_tile( const LateralParams< T >& P, unsig
                 diff[k] = T( 0 );
 #pragma unroll
                 for ( int i = 0; i < kStencil; ++i )
-                    diff[k] += f[i][OP::S + k] * ( v[i] - vb[i] );
+                    diff[k] += f[i][OP::S + k] * ( v[i] - u[( stencil_dx( i ) * ( kTileY + 2 ) + stencil_dy( i ) ) * kStride + l - 1] );
             }
             if ( above != kNeu || below != kNeu ) // a layer next to this level that does not couple its levels
             {
@@ -228,9 +251,6 @@ __device__ __forceinline__ void lateral_tile( const LateralParams< T >& P, unsig
             }
             b     = t;
             below = above;
-#pragma unroll
-            for ( int i = 0; i < kStencil; ++i )
-                vb[i] = v[i];
         }
         if ( rb == n1 )
             o[P.N] = high;
@@ -244,16 +264,34 @@ __device__ __forceinline__ void lateral_tile( const LateralParams< T >& P, unsig
         {
             T*       g = dst + size_t( cx ) * n1 * n1 + ra + hl;
             const T* c = out + cx * kTileY * kStride + hl;
+            if constexpr ( CG ) // interior columns are owned
+            {
+                T*       q = cg.p_new + ( g - P.dst.p[0] );
+                const T* v = in + ( ( cx + 1 ) * ( kTileY + 2 ) + 1 ) * kStride + hl + 1;
+                double   part[2] = { 0.0, 0.0 }; // plain sums per thread (two chains), compensated across threads
 #pragma unroll
-            for ( int cy = 0; cy < kTileY; ++cy, g += n1 )
-                if ( cy < ymax )
-                    *g = P.add ? *g + c[cy * kStride] : c[cy * kStride];
+                for ( int cy = 0; cy < kTileY; ++cy, g += n1, q += n1 )
+                    if ( cy < ymax && cg.live )
+                    {
+                        *g = c[cy * kStride];
+                        *q = v[cy * kStride];
+                        part[cy & 1] += c[cy * kStride] * v[cy * kStride];
+                    }
+                dot.add( part[0] + part[1] );
+            }
+            else
+            {
+#pragma unroll
+                for ( int cy = 0; cy < kTileY; ++cy, g += n1 )
+                    if ( cy < ymax )
+                        *g = P.add ? *g + c[cy * kStride] : c[cy * kStride];
+            }
         }
     }
 }
 
-template < typename OP, typename T >
-__device__ __forceinline__ void lateral_edge( const LateralParams< T >& P, unsigned block )
+template < typename OP, bool CG, typename T >
+__device__ __forceinline__ void lateral_edge( const LateralParams< T >& P, const LateralCG& cg, T beta, unsigned block, Neumaier& dot )
 {
     constexpr int  K = OP::K, R = OP::R;
     const int      n1 = P.n1, N = P.N;
@@ -275,19 +313,33 @@ __device__ __forceinline__ void lateral_edge( const LateralParams< T >& P, unsig
 #pragma unroll
     for ( int k = 0; k < K; ++k )
         s[1].self[k] = T( 0 );
+    T owner = T( 0 ); // the direction at the owning (first) copy
+    // value of stored node i: of the field, or of the new direction
+    const auto value = [&]( ptrdiff_t i ) {
+        if constexpr ( CG )
+            return cg.r[i] + beta * src[i];
+        else
+            return src[i];
+    };
     for ( int m = m0; m < m1; ++m )
     {
-        const int col = P.members[m], y = col % n1, x = col / n1 % n1;
-        const T*  u   = src + size_t( col ) * n1 + r;
-        const T   v0[3] = { u[rd], u[0], u[ru] };
+        const int       col = P.members[m], y = col % n1, x = col / n1 % n1;
+        const ptrdiff_t u = ptrdiff_t( col ) * n1 + r;
+        const T         v0[3] = { value( u + rd ), value( u ), value( u + ru ) };
+        if constexpr ( CG )
+        {
+            if ( cg.live )
+                cg.p_new[u] = v0[1];
+            owner = m == m0 ? v0[1] : owner;
+        }
 #pragma unroll
         for ( int i = 0; i < kStencil; ++i )
         {
             const int dx = stencil_dx( i ), dy = stencil_dy( i );
             if ( x + dx < 0 || x + dx > N || y + dy < 0 || y + dy > N )
                 continue; // no triangle of this diamond there
-            const T* q = u + ptrdiff_t( dx * n1 + dy ) * n1;
-            const T  v[3] = { q[rd], q[0], q[ru] };
+            const ptrdiff_t q = u + ptrdiff_t( dx * n1 + dy ) * n1;
+            const T         v[3] = { i ? value( q + rd ) : v0[0], i ? value( q ) : v0[1], i ? value( q + ru ) : v0[2] };
 #pragma unroll
             for ( int k = 0; k < K; ++k )
             {
@@ -327,11 +379,15 @@ __device__ __forceinline__ void lateral_edge( const LateralParams< T >& P, unsig
         lateral_layer< OP >( layer_mode( r - 1, N, P.mode_first, P.mode_inner, P.mode_last ), fr, s[0], s[1], diff[0], low, high );
         v += high;
     }
+    if constexpr ( CG )
+        dot.add( owner * v );
     T* dst = P.dst.at( blockIdx.y );
     for ( int m = m0; m < m1; ++m )
     {
         T* p = dst + size_t( P.members[m] ) * n1 + r;
-        *p   = P.add ? *p + v : v;
+        if ( CG && !cg.live )
+            break;
+        *p = P.add ? *p + v : v;
     }
 }
 
@@ -347,10 +403,11 @@ __global__ void __launch_bounds__( kLateralThreads, 4 ) lateral_kernel( LateralP
 {
     extern __shared__ double lateral_smem[];
     T*                       smem = reinterpret_cast< T* >( lateral_smem );
+    Neumaier                 none;
     if ( blockIdx.x < P.edge_blocks )
-        lateral_edge< OP >( P, blockIdx.x );
+        lateral_edge< OP, false >( P, LateralCG{}, T( 0 ), blockIdx.x, none );
     else
-        lateral_tile< OP >( P, blockIdx.x - P.edge_blocks, smem );
+        lateral_tile< OP, false >( P, LateralCG{}, T( 0 ), blockIdx.x - P.edge_blocks, smem, none );
 }
 
 // Launches lateral_kernel for every node of nc fields; Replace with additive communication merges the copies, Add
@@ -358,34 +415,50 @@ __global__ void __launch_bounds__( kLateralThreads, 4 ) lateral_kernel( LateralP
 template < typename T >
 int halo_sum( const tn_mesh* m, T* const* fields, int nfields, cudaStream_t st );
 
-template < typename OP, typename T >
-int launch_lateral( const tn_mesh* m, LateralParams< T > P, int nc, int apply_mode, int comm_mode, cudaStream_t st )
+// fills the launch shape of P (merge: the copies of a column are summed and all written) and returns its blocks
+template < typename T >
+unsigned lateral_shape( const tn_mesh* m, bool merge, LateralParams< T >& P )
 {
     P.N = m->N, P.n1 = m->n1, P.columns = m->nlat;
-    P.add = apply_mode == TN_APPLY_ADD;
-    const bool merge = !P.add && comm_mode == TN_COMM_ADDITIVE;
     P.tiles_x = ( m->N - 1 + kTileX - 1 ) / kTileX, P.tiles_y = ( m->N - 1 + kTileY - 1 ) / kTileY;
     const unsigned tiles = unsigned( m->nd ) * unsigned( P.tiles_x * P.tiles_y );
     // runs of at most kMaxRun levels; shorter ones (down to 8) while they leave SMs without a block
     P.runs = ( m->n1 + kMaxRun - 1 ) / kMaxRun;
     while ( tiles * unsigned( P.runs ) < 2u * 148u && m->n1 > 8 * P.runs )
         ++P.runs;
-    P.run        = ( m->n1 + P.runs - 1 ) / P.runs;
-    P.runs       = ( m->n1 + P.run - 1 ) / P.run;
-    P.members    = m->d_halo_members;
-    P.offsets    = merge ? m->d_halo_offsets : nullptr;
-    P.edge_nodes = unsigned( merge ? m->n_halo_groups : m->n_halo_members ) * unsigned( m->n1 );
+    P.run         = ( m->n1 + P.runs - 1 ) / P.runs;
+    P.runs        = ( m->n1 + P.run - 1 ) / P.run;
+    P.members     = m->d_halo_members;
+    P.offsets     = merge ? m->d_halo_offsets : nullptr;
+    P.edge_nodes  = unsigned( merge ? m->n_halo_groups : m->n_halo_members ) * unsigned( m->n1 );
     P.edge_blocks = ( P.edge_nodes + kLateralThreads - 1 ) / kLateralThreads;
-    constexpr size_t smem = sizeof( T ) * lateral_words< OP >();
-    static std::atomic< bool > opted_in[kMaxDevices];
-    const int                  dev = current_device();
-    if ( !opted_in[dev].load( std::memory_order_acquire ) )
+    return P.edge_blocks + tiles * unsigned( P.runs );
+}
+
+// allows `kernel` the shared memory of a tile block, once per device
+template < typename OP, typename T, typename F >
+int lateral_opt_in( std::atomic< bool > ( &done )[kMaxDevices], F* kernel )
+{
+    const int dev = current_device();
+    if ( !done[dev].load( std::memory_order_acquire ) )
     {
-        TN_CUDA_TRY( cudaFuncSetAttribute( lateral_kernel< OP, T >, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           int( smem ) ) );
-        opted_in[dev].store( true, std::memory_order_release );
+        TN_CUDA_TRY( cudaFuncSetAttribute( kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           int( sizeof( T ) * lateral_words< OP >() ) ) );
+        done[dev].store( true, std::memory_order_release );
     }
-    lateral_kernel< OP, T ><<< dim3( P.edge_blocks + tiles * unsigned( P.runs ), unsigned( nc ) ), kLateralThreads, smem, st >>>( P );
+    return TN_OK;
+}
+
+template < typename OP, typename T >
+int launch_lateral( const tn_mesh* m, LateralParams< T > P, int nc, int apply_mode, int comm_mode, cudaStream_t st )
+{
+    P.add = apply_mode == TN_APPLY_ADD;
+    const bool     merge  = !P.add && comm_mode == TN_COMM_ADDITIVE;
+    const unsigned blocks = lateral_shape( m, merge, P );
+    static std::atomic< bool > opted_in[kMaxDevices];
+    if ( const int rc = lateral_opt_in< OP, T >( opted_in, lateral_kernel< OP, T > ) )
+        return rc;
+    lateral_kernel< OP, T ><<< dim3( blocks, unsigned( nc ) ), kLateralThreads, sizeof( T ) * lateral_words< OP >(), st >>>( P );
     TN_LAUNCH_CHECK();
     if ( !merge && comm_mode == TN_COMM_ADDITIVE )
         return halo_sum< T >( m, P.dst.p, nc, st );

@@ -9,7 +9,7 @@
 // and a radial factor (MassOp, lateral.cuh).  With a nodal k, and lumped: one
 // thread per cell, atomic accumulation, then the additive halo (setup work).
 #include "common.cuh"
-#include "lateral.cuh"
+#include "lateral_cg.cuh"
 #include "wedge.cuh"
 
 namespace tn {
@@ -118,7 +118,7 @@ struct MassOp
         for ( int q = 0; q < 3; ++q )
         {
             const double l[3] = { 1.0 - kMQP[q][0] - kMQP[q][1], kMQP[q][0], kMQP[q][1] };
-            A[0] += 0.1666666666666667 * fabs( D ) * l[i] * l[j];
+            A[0] += fabs( D ) * l[i] * l[j] / 6.0;
         }
     }
     static __device__ void radial( double r1, double r2, double* f )
@@ -167,6 +167,27 @@ int kmass_apply( const tn_mesh* m, const T* k, int mode, int apply_mode, int com
         return halo_sum< T >( m, f, 1, st );
     }
     return TN_OK;
+}
+
+// CG on the plain mass matrix from x's values (lateral_cg.cuh); fields: 4 stored-node fields
+int mass_cg( const tn_mesh* m, const double* b, double* x, double* fields, int max_iterations, double rtol, double atol,
+             int* iterations, cudaStream_t st )
+{
+    LateralParams< double > P{};
+    if ( !lateral_tables< MassOp< double > >( m, &tn_mesh::mass_tables, P, st ) )
+    {
+        set_error( "mass_cg: allocating the lateral stencil failed" );
+        return TN_ERR_NOMEM;
+    }
+    const size_t    ns = m->ns;
+    const WorkBlock w( m, lateral_cg_scratch< MassOp< double > >( m, max_iterations ) );
+    if ( !w.get() )
+    {
+        set_error( "mass_cg: allocating the scratch failed" );
+        return TN_ERR_NOMEM;
+    }
+    double* const f[4] = { fields, fields + ns, fields + 2 * ns, fields + 3 * ns };
+    return lateral_cg< MassOp< double > >( m, P, b, x, f, w.get(), max_iterations, rtol, atol, iterations, nullptr, st );
 }
 
 template int kmass_apply< double >( const tn_mesh*, const double*, int, int, int, const double*, double*, cudaStream_t );

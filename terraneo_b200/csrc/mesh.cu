@@ -158,6 +158,38 @@ int halo_sum( const tn_mesh* m, T* const* fields, int nfields, cudaStream_t st )
 template int halo_sum< double >( const tn_mesh*, double* const*, int, cudaStream_t );
 template int halo_sum< float >( const tn_mesh*, float* const*, int, cudaStream_t );
 
+WorkBlock::WorkBlock( const tn_mesh* m, size_t n ) : m_( const_cast< tn_mesh* >( m ) ), n_( n )
+{
+    {
+        std::lock_guard< std::mutex > lock( m_->work_mutex );
+        if ( m_->d_work && m_->n_work >= n )
+        {
+            p_ = m_->d_work, n_ = m_->n_work;
+            m_->d_work = nullptr, m_->n_work = 0;
+        }
+    }
+    if ( !p_ && cudaMalloc( &p_, n * sizeof( double ) ) != cudaSuccess )
+    {
+        (void) cudaGetLastError();
+        p_ = nullptr;
+    }
+}
+
+WorkBlock::~WorkBlock()
+{
+    if ( !p_ )
+        return;
+    {
+        std::lock_guard< std::mutex > lock( m_->work_mutex );
+        if ( n_ > m_->n_work )
+        {
+            std::swap( p_, m_->d_work );
+            std::swap( n_, m_->n_work );
+        }
+    }
+    cudaFree( p_ );
+}
+
 // a b - c d with the rounding error of c d put back (Kahan's difference of products: within 1.5 ulp)
 __device__ __forceinline__ double diff_of_products( double a, double b, double c, double d )
 {
@@ -474,6 +506,7 @@ extern "C" int tn_mesh_destroy( tn_mesh* m )
         cudaFree( t->lat32 );
         cudaFree( t->rad32 );
     }
+    cudaFree( m->d_work );
     cudaFree( m->d_triangles );
     cudaFree( m->d_red_partials );
     cudaFree( m->d_red_result );

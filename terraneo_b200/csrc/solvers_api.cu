@@ -17,6 +17,11 @@
 #include "../cpp/tn/solvers.hpp"
 #include "common.cuh"
 
+namespace tn {
+int laplace_cg( const tn_mesh* m, const double* b, double* x, int max_iterations, double rtol, double atol, int* iterations,
+                double* relres, cudaStream_t st );
+}
+
 using namespace tn;
 
 namespace {
@@ -757,30 +762,12 @@ extern "C" int tn_laplace_pcg_solve_f64( const tn_mesh* mesh, const double* b, d
                                          double* relative_residual )
 {
     TN_CHECK_ARG( mesh && b && x, "tn_laplace_pcg_solve_f64: null argument" );
-    try
-    {
-        Mesh                     m = Mesh::wrap( mesh );
-        Laplace< double >        A( m, true, false );
-        VectorQ1Scalar< double > vb( m, const_cast< double* >( b ) ), vx( m, x );
-        std::vector< VectorQ1Scalar< double > > t;
-        for ( int i = 0; i < 3; ++i )
-            t.emplace_back( m );
-        DevicePCG< Laplace< double > > pcg(
-            IterativeSolverParameters{ max_iterations, relative_tolerance, absolute_tolerance }, t );
-        solve( pcg, A, vx, vb );
-        const SolverStatistics st = pcg.statistics();
-        TN_CUDA_TRY( cudaDeviceSynchronize() );
-        if ( iterations )
-            *iterations = st.iterations;
-        if ( relative_residual )
-            *relative_residual = st.relative_residuals.back();
-        return TN_OK;
-    }
-    catch ( const std::exception& e )
-    {
-        set_error( std::string( "tn_laplace_pcg_solve_f64: " ) + e.what() );
-        return TN_ERR_STATE;
-    }
+    const int rc = laplace_cg( mesh, b, x, max_iterations, relative_tolerance, absolute_tolerance, iterations, relative_residual,
+                               static_cast< cudaStream_t >( stream() ) );
+    if ( rc )
+        return rc;
+    TN_CUDA_TRY( cudaDeviceSynchronize() );
+    return TN_OK;
 }
 
 // The library's Krylov solver templates without a preconditioner on the scalar

@@ -20,6 +20,8 @@ namespace tn {
 
 template < typename T >
 int halo_sum( const tn_mesh* m, T* const* fields, int nfields, cudaStream_t st );
+int mass_cg( const tn_mesh* m, const double* b, double* x, double* fields, int max_iterations, double rtol, double atol,
+             int* iterations, cudaStream_t st );
 
 namespace {
 
@@ -208,32 +210,7 @@ extern "C" int tn_l2_project_fv_to_fe_f64( const tn_mesh* m, const double* src, 
     int rc = tn_fv_to_fe_rhs_f64( m, src, work, nullptr, s );
     if ( rc )
         return rc;
-    try
-    {
-        struct StreamScope // the C++ layer issues on tn::stream(): this call's stream for its duration
-        {
-            cudaStream_t prev;
-            explicit StreamScope( cudaStream_t s ) : prev( stream_ref() ) { stream_ref() = s; }
-            ~StreamScope() { stream_ref() = prev; }
-        } scope( st );
-        Mesh                              mesh = Mesh::wrap( m );
-        VectorQ1Scalar< double >          b( mesh, work ), x( mesh, dst ), none;
-        std::vector< VectorQ1Scalar< double > > tmps;
-        for ( int i = 1; i <= 4; ++i )
-            tmps.emplace_back( mesh, work + i * ns );
-        KMass< double > M( mesh, none, 0 );
-        PCG< KMass< double > > pcg( IterativeSolverParameters{ max_iterations, relative_tolerance, absolute_tolerance },
-                                    tmps );
-        solve( pcg, M, x, b );
-        if ( iterations )
-            *iterations = pcg.stats.iterations;
-    }
-    catch ( const std::exception& e )
-    {
-        set_error( std::string( "tn_l2_project_fv_to_fe_f64: " ) + e.what() );
-        return TN_ERR_CUDA;
-    }
-    return TN_OK;
+    return mass_cg( m, work, dst, work + ns, max_iterations, relative_tolerance, absolute_tolerance, iterations, st );
 }
 
 // f = VectorMass (Ra T n) with n the unit radial direction (mantlecirculation.cpp:117-150, 883-886), then the
