@@ -772,7 +772,7 @@ struct SpcgParams
     unsigned*      counter;
 };
 
-__device__ __forceinline__ void spcg_position( const SpcgParams& S, unsigned i, double xp[3] )
+__device__ __forceinline__ void spcg_position( const SpcgParams& S, unsigned i, double ( &xp )[3] )
 {
     const unsigned n1  = unsigned( S.n1 );
     const unsigned lat = i / n1; // ns < 2^32 at every level tn_mesh_create accepts (<= 9)
@@ -930,20 +930,22 @@ struct ClusterPcgParams
 {
     SpcgParams           S;
     Ptr3< const double > b;
-    Ptr3< double >       x, r, p, ap, aq;
+    Ptr3< double >       x, r, p, ap;
     int                  it; // 0: initial residual (r = b - a, p = r); >= 1: PCG iteration it
     double               rtol, atol;
 };
 
 // sum over the cluster of K compensated per-thread partials; the result is
 // the same in every thread of every CTA.  part: this CTA's partials in the
-// given slot (each slot is used once per launch).
+// given slot (each slot is used once per launch).  Warps and ranks are merged
+// as trees by warp 0 (a serial merge of 16 + 16 compensated pairs cost more
+// than the barrier).
 template < int K >
 __device__ void cluster_sum( cg::cluster_group& cl, Neumaier* acc, double ( *part )[K][2], int slot, double* out )
 {
     __shared__ double sh[32][K][2];
     __shared__ double res[K];
-    const int         lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int         lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = int( blockDim.x >> 5 );
 #pragma unroll
     for ( int k = 0; k < K; ++k )
     {
@@ -952,38 +954,29 @@ __device__ void cluster_sum( cg::cluster_group& cl, Neumaier* acc, double ( *par
             sh[warp][k][0] = w.s, sh[warp][k][1] = w.c;
     }
     __syncthreads();
-    if ( threadIdx.x == 0 )
+    if ( warp == 0 )
+#pragma unroll
         for ( int k = 0; k < K; ++k )
         {
-            Neumaier b;
-            for ( int w = 0; w < int( blockDim.x >> 5 ); ++w )
-                b.merge( Neumaier{ sh[w][k][0], sh[w][k][1] } );
-            part[slot][k][0] = b.s, part[slot][k][1] = b.c;
+            const int      j = lane < nwarps ? lane : 0;
+            const Neumaier b = merge_warps( sh[j][k][0], sh[j][k][1], lane, nwarps );
+            if ( lane == 0 )
+                part[slot][k][0] = b.s, part[slot][k][1] = b.c;
         }
     cl.sync();
     if ( warp == 0 )
     {
-        // lane j fetches rank j's partials (one round of remote loads), then
-        // every lane merges them in rank order from shuffles
-        const unsigned nb = cl.num_blocks();
-        double         qs[K], qc[K];
+        // lane j fetches rank j's partials (one round of remote loads)
+        const int     nb = int( cl.num_blocks() );
+        const double* q  = cl.map_shared_rank( &part[slot][0][0], unsigned( lane < nb ? lane : 0 ) );
+        double        qs[K], qc[K];
 #pragma unroll
         for ( int k = 0; k < K; ++k )
-            qs[k] = qc[k] = 0.0;
-        if ( unsigned( lane ) < nb )
-        {
-            const double* q = cl.map_shared_rank( &part[slot][0][0], unsigned( lane ) );
-#pragma unroll
-            for ( int k = 0; k < K; ++k )
-                qs[k] = q[2 * k], qc[k] = q[2 * k + 1];
-        }
+            qs[k] = q[2 * k], qc[k] = q[2 * k + 1];
 #pragma unroll
         for ( int k = 0; k < K; ++k )
         {
-            Neumaier t;
-            for ( unsigned j = 0; j < nb; ++j )
-                t.merge( Neumaier{ __shfl_sync( 0xffffffffu, qs[k], int( j ) ),
-                                   __shfl_sync( 0xffffffffu, qc[k], int( j ) ) } );
+            const Neumaier t = merge_warps( qs[k], qc[k], lane, nb );
             if ( lane == 0 )
                 res[k] = t.value();
         }
@@ -994,6 +987,10 @@ __device__ void cluster_sum( cg::cluster_group& cl, Neumaier* acc, double ( *par
         out[k] = res[k];
 }
 
+// PER: nodes per thread (nodes t0, t0 + nt, ...; 1 for a cluster of 16 at level 3).  A thread keeps its nodes' p, r, x,
+// A p and position in registers over the three phases, and loads them all before the first: the phases are serial, and
+// each of their reloads was an L2 round trip.  Level 3, per step: 16.0 -> 11.3 us with that and the tree merges.
+template < int PER >
 __global__ void __launch_bounds__( kCpThreads ) spcg_step_cluster_kernel( ClusterPcgParams P )
 {
     __shared__ double part3[1][3][2];
@@ -1003,52 +1000,64 @@ __global__ void __launch_bounds__( kCpThreads ) spcg_step_cluster_kernel( Cluste
     double*           st = S.state;
     if ( P.it > 0 && st[kSpDone] != 0.0 ) // uniform: read by every thread before any barrier
         return;
-    const size_t   ns   = S.ns;
-    const size_t   t0   = size_t( cl.block_rank() ) * blockDim.x + threadIdx.x;
-    const size_t   nt   = size_t( cl.num_blocks() ) * blockDim.x;
+    const unsigned ns   = unsigned( S.ns );
+    const unsigned t0   = cl.block_rank() * blockDim.x + threadIdx.x;
+    const unsigned nt   = cl.num_blocks() * blockDim.x;
     const unsigned n1   = unsigned( S.n1 );
     const bool     lead = cl.block_rank() == 0 && threadIdx.x == 0;
     const double   g[3] = { S.fsfs ? S.scratch[3] : 0.0, S.fsfs ? S.scratch[4] : 0.0, S.fsfs ? S.scratch[5] : 0.0 };
     double         an = st[kSpAn], r0 = st[kSpR0];
 
+    // q: b (it 0) or p; every load of the nodes before any store
+    double q[PER][3], rv[PER][3], xv[PER][3], a[PER][3], xp[PER][3];
+    bool   in[PER], own[PER];
+#pragma unroll
+    for ( int k = 0; k < PER; ++k )
+    {
+        const unsigned i = t0 + k * nt;
+        in[k]            = i < ns;
+        own[k]           = in[k] && S.owned[i];
+#pragma unroll
+        for ( int c = 0; c < 3; ++c )
+        {
+            q[k][c]  = in[k] ? __ldcg( ( P.it == 0 ? P.b.p[c] : P.p.p[c] ) + i ) : 0.0;
+            rv[k][c] = in[k] && P.it > 0 ? __ldcg( P.r.p[c] + i ) : 0.0;
+            xv[k][c] = in[k] && P.it > 0 ? __ldcg( P.x.p[c] + i ) : 0.0;
+            xp[k][c] = 0.0;
+        }
+        if ( S.fsfs && in[k] )
+            spcg_position( S, i, xp[k] );
+    }
     // a = halo sum over the node's copies of (ap + g x x); it 0: r = b - a,
-    // p = r and <r, r>; else aq = a and <p, aq>
+    // p = r and <r, r>; else <p, a>
     double red;
     {
         Neumaier acc;
-        for ( size_t i = t0; i < ns; i += nt )
-        {
-            double pen[3] = { 0.0, 0.0, 0.0 };
-            if ( S.fsfs )
-            {
-                double xp[3];
-                spcg_position( S, unsigned( i ), xp );
-                pen[0] = g[1] * xp[2] - g[2] * xp[1];
-                pen[1] = g[2] * xp[0] - g[0] * xp[2];
-                pen[2] = g[0] * xp[1] - g[1] * xp[0];
-            }
-            const unsigned lat = unsigned( i ) / n1, rr = unsigned( i ) - lat * n1;
-            const int      grp = S.lat_group[lat];
-            // every load of the node before any store (the fields may alias as far as the compiler knows)
-            double a[3], q[3];
 #pragma unroll
-            for ( int c = 0; c < 3; ++c )
-                q[c] = __ldcg( ( P.it == 0 ? P.b.p[c] : P.p.p[c] ) + i );
+        for ( int k = 0; k < PER; ++k )
+        {
+            const unsigned i = t0 + k * nt;
+            if ( !in[k] )
+                continue;
+            const double   pen[3] = { g[1] * xp[k][2] - g[2] * xp[k][1], g[2] * xp[k][0] - g[0] * xp[k][2],
+                                      g[0] * xp[k][1] - g[1] * xp[k][0] };
+            const unsigned lat = i / n1, rr = i - lat * n1;
+            const int      grp = S.lat_group[lat];
             if ( grp < 0 )
             {
 #pragma unroll
                 for ( int c = 0; c < 3; ++c )
-                    a[c] = __ldcg( P.ap.p[c] + i ) + pen[c];
+                    a[k][c] = __ldcg( P.ap.p[c] + i ) + pen[c];
             }
             else
             {
-                a[0] = a[1] = a[2] = 0.0;
-                for ( int k = S.offsets[grp]; k < S.offsets[grp + 1]; ++k )
+                a[k][0] = a[k][1] = a[k][2] = 0.0;
+                for ( int m = S.offsets[grp]; m < S.offsets[grp + 1]; ++m )
                 {
-                    const size_t j = size_t( S.members[k] ) * n1 + rr;
+                    const size_t j = size_t( S.members[m] ) * n1 + rr;
 #pragma unroll
                     for ( int c = 0; c < 3; ++c )
-                        a[c] += __ldcg( P.ap.p[c] + j ) + pen[c];
+                        a[k][c] += __ldcg( P.ap.p[c] + j ) + pen[c];
                 }
             }
             double dot = 0.0;
@@ -1057,18 +1066,15 @@ __global__ void __launch_bounds__( kCpThreads ) spcg_step_cluster_kernel( Cluste
             {
                 if ( P.it == 0 )
                 {
-                    const double ri = q[c] - a[c];
-                    __stcg( P.r.p[c] + i, ri );
-                    __stcg( P.p.p[c] + i, ri );
-                    dot += ri * ri;
+                    q[k][c] -= a[k][c];
+                    __stcg( P.r.p[c] + i, q[k][c] );
+                    __stcg( P.p.p[c] + i, q[k][c] );
+                    dot += q[k][c] * q[k][c];
                 }
                 else
-                {
-                    __stcg( P.aq.p[c] + i, a[c] );
-                    dot += q[c] * a[c];
-                }
+                    dot += q[k][c] * a[k][c];
             }
-            acc.add( S.owned[i] ? dot : 0.0 );
+            acc.add( own[k] ? dot : 0.0 );
         }
         cluster_sum< 1 >( cl, &acc, part1, 0, &red );
     }
@@ -1087,29 +1093,27 @@ __global__ void __launch_bounds__( kCpThreads ) spcg_step_cluster_kernel( Cluste
     }
     else
     {
-        // x += alpha p, r -= alpha aq, <r, r>, stopping test  (pcg.hpp:88-110)
+        // x += alpha p, r -= alpha ap, <r, r>, stopping test  (pcg.hpp:88-110)
         const double pap = red, alpha = an / pap;
         double       rr;
         {
             Neumaier acc;
-            for ( size_t i = t0; i < ns; i += nt )
+#pragma unroll
+            for ( int k = 0; k < PER; ++k )
             {
-                double xv[3], pv[3], rv[3], qv[3], dot = 0.0;
+                const unsigned i = t0 + k * nt;
+                if ( !in[k] )
+                    continue;
+                double dot = 0.0;
 #pragma unroll
                 for ( int c = 0; c < 3; ++c )
                 {
-                    xv[c] = __ldcg( P.x.p[c] + i ), pv[c] = __ldcg( P.p.p[c] + i );
-                    rv[c] = __ldcg( P.r.p[c] + i ), qv[c] = __ldcg( P.aq.p[c] + i );
+                    __stcg( P.x.p[c] + i, xv[k][c] + alpha * q[k][c] );
+                    rv[k][c] += ( -alpha ) * a[k][c];
+                    __stcg( P.r.p[c] + i, rv[k][c] );
+                    dot += rv[k][c] * rv[k][c];
                 }
-#pragma unroll
-                for ( int c = 0; c < 3; ++c )
-                {
-                    __stcg( P.x.p[c] + i, xv[c] + alpha * pv[c] );
-                    const double ri = rv[c] + ( -alpha ) * qv[c];
-                    __stcg( P.r.p[c] + i, ri );
-                    dot += ri * ri;
-                }
-                acc.add( S.owned[i] ? dot : 0.0 );
+                acc.add( own[k] ? dot : 0.0 );
             }
             cluster_sum< 1 >( cl, &acc, part1, 1, &rr );
         }
@@ -1131,32 +1135,27 @@ __global__ void __launch_bounds__( kCpThreads ) spcg_step_cluster_kernel( Cluste
         // next direction p = r + beta p (p = r after the initial residual),
         // ap = 0, penalty dots of p and g = eps G^-1 d for the next apply
         double sum[3] = { 0.0, 0.0, 0.0 };
-        for ( size_t i = t0; i < ns; i += nt )
-        {
-            double w[3], rv[3];
 #pragma unroll
-            for ( int c = 0; c < 3; ++c )
-            {
-                w[c]  = __ldcg( P.p.p[c] + i );
-                rv[c] = P.it > 0 ? __ldcg( P.r.p[c] + i ) : 0.0;
-            }
+        for ( int k = 0; k < PER; ++k )
+        {
+            const unsigned i = t0 + k * nt;
+            if ( !in[k] )
+                continue;
 #pragma unroll
             for ( int c = 0; c < 3; ++c )
             {
                 if ( P.it > 0 )
                 {
-                    w[c] = rv[c] + beta * w[c];
-                    __stcg( P.p.p[c] + i, w[c] );
+                    q[k][c] = rv[k][c] + beta * q[k][c];
+                    __stcg( P.p.p[c] + i, q[k][c] );
                 }
                 __stcg( P.ap.p[c] + i, 0.0 );
             }
-            if ( S.fsfs && S.owned[i] )
+            if ( own[k] ) // the position is zero without the penalty
             {
-                double xp[3];
-                spcg_position( S, unsigned( i ), xp );
-                sum[0] += xp[1] * w[2] - xp[2] * w[1];
-                sum[1] += xp[2] * w[0] - xp[0] * w[2];
-                sum[2] += xp[0] * w[1] - xp[1] * w[0];
+                sum[0] += xp[k][1] * q[k][2] - xp[k][2] * q[k][1];
+                sum[1] += xp[k][2] * q[k][0] - xp[k][0] * q[k][2];
+                sum[2] += xp[k][0] * q[k][1] - xp[k][1] * q[k][0];
             }
         }
         if ( S.fsfs )
@@ -1188,8 +1187,10 @@ int spcg_cluster_size()
         return size;
     known[dev] = true;
     size       = 0;
-    if ( cudaFuncSetAttribute( spcg_step_cluster_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1 ) !=
-         cudaSuccess )
+    if ( cudaFuncSetAttribute( spcg_step_cluster_kernel< 1 >, cudaFuncAttributeNonPortableClusterSizeAllowed, 1 ) !=
+             cudaSuccess ||
+         cudaFuncSetAttribute( spcg_step_cluster_kernel< 2 >, cudaFuncAttributeNonPortableClusterSizeAllowed, 1 ) !=
+             cudaSuccess )
     {
         cudaGetLastError();
         return size;
@@ -1202,7 +1203,7 @@ int spcg_cluster_size()
         attr.val.clusterDim.x = unsigned( c ), attr.val.clusterDim.y = 1, attr.val.clusterDim.z = 1;
         cfg.gridDim = dim3( unsigned( c ) ), cfg.blockDim = dim3( kCpThreads ), cfg.attrs = &attr, cfg.numAttrs = 1;
         int n = 0;
-        if ( cudaOccupancyMaxActiveClusters( &n, spcg_step_cluster_kernel, &cfg ) == cudaSuccess && n >= 1 )
+        if ( cudaOccupancyMaxActiveClusters( &n, spcg_step_cluster_kernel< 2 >, &cfg ) == cudaSuccess && n >= 1 )
         {
             size = c;
             break;
@@ -1314,13 +1315,17 @@ static int stored_pcg( const tn_mesh* m, const double* mats, const tn_epsdivdiv_
     cudaLaunchAttribute attr{};
     if ( csize > 0 )
     {
-        CP.S = S, CP.b = pb, CP.x = px, CP.r = pr, CP.p = pp, CP.ap = pap, CP.aq = paq;
+        CP.S = S, CP.b = pb, CP.x = px, CP.r = pr, CP.p = pp, CP.ap = pap;
         CP.rtol = rtol, CP.atol = atol;
         attr.id               = cudaLaunchAttributeClusterDimension;
         attr.val.clusterDim.x = unsigned( csize ), attr.val.clusterDim.y = 1, attr.val.clusterDim.z = 1;
         cfg.gridDim = dim3( unsigned( csize ) ), cfg.blockDim = dim3( kCpThreads ), cfg.dynamicSmemBytes = 0;
         cfg.stream = st, cfg.attrs = &attr, cfg.numAttrs = 1;
     }
+
+    // nodes per thread of the cluster: 7,290 at level 3, so 1 with 16 CTAs of 512 threads and 2 with 8
+    const auto cluster_step =
+        m->ns <= size_t( std::max( csize, 1 ) ) * kCpThreads ? spcg_step_cluster_kernel< 1 > : spcg_step_cluster_kernel< 2 >;
 
     // r = b - A x, p = r
     spcg_prepare_kernel<<< nblocks, 256, 0, st >>>( S, pp, cr, cx, pap, 0, 0 );
@@ -1332,7 +1337,7 @@ static int stored_pcg( const tn_mesh* m, const double* mats, const tn_epsdivdiv_
     {
         // also clears ap and forms the penalty vector of p for the first iteration
         CP.it = 0;
-        TN_CUDA_TRY( cudaLaunchKernelEx( &cfg, spcg_step_cluster_kernel, CP ) );
+        TN_CUDA_TRY( cudaLaunchKernelEx( &cfg, cluster_step, CP ) );
     }
     else
         spcg_gather_kernel<<< nblocks, 256, 0, st >>>( S, cap, 0, pb, pr, pp, paq, atol );
@@ -1358,7 +1363,7 @@ static int stored_pcg( const tn_mesh* m, const double* mats, const tn_epsdivdiv_
             stored_apply_kernel< double ><<< ablocks, 128, 0, st >>>( A );
             TN_LAUNCH_CHECK();
             CP.it = it;
-            TN_CUDA_TRY( cudaLaunchKernelEx( &cfg, spcg_step_cluster_kernel, CP ) );
+            TN_CUDA_TRY( cudaLaunchKernelEx( &cfg, cluster_step, CP ) );
             TN_LAUNCH_CHECK();
             continue;
         }

@@ -41,6 +41,13 @@ __device__ __forceinline__ Neumaier warp_reduce( Neumaier a )
     return a;
 }
 
+// sum of the warps' sums of a block (n <= 32 of them) by warp 0: lane j brings warp j's, merged as a tree (five
+// dependent merges instead of one per warp; the order is still fixed)
+__device__ __forceinline__ Neumaier merge_warps( double s, double c, int lane, int n )
+{
+    return warp_reduce( lane < n ? Neumaier{ s, c } : Neumaier{} );
+}
+
 // Reduces K compensated sums over the whole grid; result[k] = total k.
 // Requires blockDim.x to be a multiple of 32 and <= 1024.  Returns true in
 // the last block (where thread 0 has just written `result`), false elsewhere.
@@ -58,19 +65,25 @@ __device__ bool block_sum_finish( Neumaier* acc, double* partials, unsigned int*
             sh_s[warp][k] = w.s, sh_c[warp][k] = w.c;
     }
     __syncthreads();
-    if ( threadIdx.x == 0 )
+    if ( warp == 0 )
     {
+#pragma unroll
         for ( int k = 0; k < K; ++k )
         {
-            Neumaier b;
-            for ( int w = 0; w < nwarps; ++w )
-                b.merge( Neumaier{ sh_s[w][k], sh_c[w][k] } );
-            partials[( size_t( blockIdx.x ) * K + k ) * 2]     = b.s;
-            partials[( size_t( blockIdx.x ) * K + k ) * 2 + 1] = b.c;
+            const int      j = lane < nwarps ? lane : 0;
+            const Neumaier b = merge_warps( sh_s[j][k], sh_c[j][k], lane, nwarps );
+            if ( lane == 0 )
+            {
+                partials[( size_t( blockIdx.x ) * K + k ) * 2]     = b.s;
+                partials[( size_t( blockIdx.x ) * K + k ) * 2 + 1] = b.c;
+            }
         }
-        __threadfence();
-        const unsigned ticket = atomicAdd( counter, 1u );
-        is_last               = ( ticket == gridDim.x - 1 );
+        if ( lane == 0 )
+        {
+            __threadfence();
+            const unsigned ticket = atomicAdd( counter, 1u );
+            is_last               = ( ticket == gridDim.x - 1 );
+        }
     }
     __syncthreads();
     if ( !is_last )
@@ -110,16 +123,18 @@ __device__ bool block_sum_finish( Neumaier* acc, double* partials, unsigned int*
             sh_s[warp][k] = w.s, sh_c[warp][k] = w.c;
     }
     __syncthreads();
-    if ( threadIdx.x == 0 )
+    if ( warp == 0 )
     {
+#pragma unroll
         for ( int k = 0; k < K; ++k )
         {
-            Neumaier b;
-            for ( int w = 0; w < nwarps; ++w )
-                b.merge( Neumaier{ sh_s[w][k], sh_c[w][k] } );
-            result[k] = b.value();
+            const int      j = lane < nwarps ? lane : 0;
+            const Neumaier b = merge_warps( sh_s[j][k], sh_c[j][k], lane, nwarps );
+            if ( lane == 0 )
+                result[k] = b.value();
         }
-        *counter = 0u;
+        if ( lane == 0 )
+            *counter = 0u;
     }
     return true;
 }
