@@ -169,6 +169,19 @@ int kmass_apply( const tn_mesh* m, const T* k, int mode, int apply_mode, int com
     return TN_OK;
 }
 
+// The stencils of the plain mass matrix, both precisions, with the mesh: its apply had no table before it was
+// separated, so a first one may not allocate or wait (it may be inside a stream capture).
+int build_mass_tables( tn_mesh* m )
+{
+    LateralParams< double > P{};
+    LateralParams< float >  Q{};
+    if ( lateral_tables< MassOp< double > >( m, &tn_mesh::mass_tables, P, nullptr ) &&
+         lateral_tables< MassOp< float > >( m, &tn_mesh::mass_tables, Q, nullptr ) )
+        return TN_OK;
+    set_error( "tn_mesh_create: allocating the lateral stencils of the mass matrix failed" );
+    return TN_ERR_NOMEM;
+}
+
 // CG on the plain mass matrix from x's values (lateral_cg.cuh); fields: 4 stored-node fields
 int mass_cg( const tn_mesh* m, const double* b, double* x, double* fields, int max_iterations, double rtol, double atol,
              int* iterations, cudaStream_t st )

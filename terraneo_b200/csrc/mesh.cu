@@ -244,6 +244,8 @@ __global__ void triangle_kernel( int N, size_t triangles, const double* __restri
     }
 }
 
+int build_mass_tables( tn_mesh* m ); // mass.cu
+
 // both tables of cell.cuh, complete for every stream on return
 int build_triangle_tables( tn_mesh* m )
 {
@@ -450,7 +452,8 @@ int mesh_create_diamonds( const ShellTopology& t, double r_min, double r_max, in
          ( rc = upload( offsets.data(), offsets.size(), &m->d_halo_offsets ) ) ||
          ( nd == kDiamonds && ( rc = upload( t.fv_ghost.data(), t.fv_ghost.size(), &m->d_fv_ghost ) ) ) ||
          ( rc = upload( members.data(), members.size(), &m->d_halo_members ) ) ||
-         ( rc = upload( lat_group.data(), lat_group.size(), &m->d_lat_group ) ) || ( rc = build_triangle_tables( m ) ) )
+         ( rc = upload( lat_group.data(), lat_group.size(), &m->d_lat_group ) ) || ( rc = build_triangle_tables( m ) ) ||
+         ( rc = build_mass_tables( m ) ) )
     {
         tn_mesh_destroy( m );
         return rc;

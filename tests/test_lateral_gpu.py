@@ -49,3 +49,19 @@ def test_every_copy_and_mode(op, bc, L, dtype, tol):
     assert rel(halo(own), ref.reshape(u.shape)) <= tol
     assert rel(_apply(*args, C.APPLY_ADD, C.COMM_SKIP), own + old) <= tol
     assert rel(_apply(*args, C.APPLY_ADD, C.COMM_ADDITIVE), halo(own + old)) <= tol
+
+
+def test_first_mass_apply_in_a_capture():
+    """nothing is allocated or waited for on a mesh's first mass apply, so it may be part of a graph"""
+    from terraneo_b200 import shell
+    pm, warm = shell.ShellMesh(3), shell.ShellMesh(2)
+    shell.apply(shell.KMass(warm), *(shell.VectorQ1Scalar(warm) for _ in range(2)))  # the module is loaded outside
+    src, dst, ref = (shell.VectorQ1Scalar(pm) for _ in range(3))
+    src.data.uniform_()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        shell.apply(shell.KMass(pm), src, dst)
+    graph.replay()
+    shell.apply(shell.KMass(pm), src, ref)
+    torch.cuda.synchronize()
+    assert torch.equal(dst.data, ref.data)
