@@ -167,8 +167,9 @@ __device__ __forceinline__ void kgrad_boundary( const KGradParams< T >& P )
         atomicAdd( P.out + id[n % 3] + n / 3, cw );
 }
 
+// Blocks per SM, level 6: FP64 at 3 / 4 / 5 blocks 128 / 134 / 155 us, FP32 at 4 / 6 89 / 86 us.
 template < typename T >
-__global__ void __launch_bounds__( 128, 4 ) kgrad_kernel( KGradParams< T > P )
+__global__ void __launch_bounds__( 128, sizeof( T ) == 8 ? 3 : 6 ) kgrad_kernel( KGradParams< T > P )
 {
     if ( blockIdx.x < P.edge_blocks )
     {

@@ -198,8 +198,10 @@ __device__ __forceinline__ void epsdivdiv_diagonal( const E32Params< T >& P, int
             atomicAdd( P.dst.p[c] + id[m] + top, o[m][c] * P.src.p[c][id[m] + top] );
 }
 
+// Blocks per SM, level 6: FP64 at 3 / 4 / 5 blocks 248 / 252 / 319 us (spills from 4 on), FP32 at 4 / 5 / 6 165 / 155 /
+// 153 us.
 template < typename T >
-__global__ void __launch_bounds__( 128, 4 ) epsdivdiv3x2_kernel( E32Params< T > P )
+__global__ void __launch_bounds__( 128, sizeof( T ) == 8 ? 3 : 6 ) epsdivdiv3x2_kernel( E32Params< T > P )
 {
     const int N = P.N, n1 = P.n1;
     int       d, x, y, r;

@@ -38,7 +38,7 @@ struct DivKGradParams
 // moments of (flux . v) over the points, all through the six scalar products of
 // beta_1, beta_2, v: about 150 multiply-adds per wedge (470 when the symmetric
 // 6 x 6 matrix is formed from a table of 63 lateral factors per wedge).
-// Apply with its halo, FP64: 330 -> 96 us at level 6, 2,562 -> 675 us at level 7;
+// Apply with its halo, FP64: 330 -> 91 us at level 6, 2,562 -> 642 us at level 7;
 // bound by instruction issue (56 % of the slots).
 template < typename T, bool SINGLE >
 __device__ __forceinline__ void divkgrad_wedge( const Triangle< T >& G, T h, T rho_m, const T ( &s )[6], const T ( &kn )[6],
@@ -143,9 +143,10 @@ __device__ __forceinline__ void divkgrad_diagonal( const DivKGradParams< T >& P,
 // One thread per cell (r fastest), contributions added by add_column.  With the
 // boundary treatment the CMB nodes of layer 0 (otherwise the SURFACE nodes of
 // layer N - 1) enter with zero and keep their diagonal, which further blocks of the
-// launch add (one thread per lateral cell, wedge and side).
+// launch add (one thread per lateral cell, wedge and side).  Blocks per SM, FP64: at 4 / 5 / 6 95 / 91 / 97 us at
+// level 6, 689 / 642 / 670 us at level 7.
 template < typename T, bool SINGLE >
-__global__ void __launch_bounds__( 128, 4 ) divkgrad_kernel( DivKGradParams< T > P )
+__global__ void __launch_bounds__( 128, 5 ) divkgrad_kernel( DivKGradParams< T > P )
 {
     const int N = P.N, n1 = P.n1;
     int       d, x, y, r;

@@ -222,8 +222,10 @@ __device__ __forceinline__ void supg_diagonal( const SupgParams< T >& P, int d, 
         atomicAdd( P.dst + id[m] + top, ( o[m] + tau * b[m] ) * P.src[id[m] + top] );
 }
 
+// Blocks per SM, level 6: FP64 at 3 / 4 / 5 blocks 459 / 456 / 604 us (level 5: 71 / 74 / 88), FP32 at 3 / 4 / 6 237 /
+// 207 / 230 us.
 template < typename T >
-__global__ void __launch_bounds__( 128, 3 ) supg_kernel( SupgParams< T > P )
+__global__ void __launch_bounds__( 128, sizeof( T ) == 8 ? 3 : 4 ) supg_kernel( SupgParams< T > P )
 {
     const int N = P.N, n1 = P.n1;
     int       d, x, y, r;
