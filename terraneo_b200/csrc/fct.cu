@@ -7,11 +7,11 @@
 // ghosts are copies of the real cells across each diamond face (the mesh's
 // FV ghost map); radial ghosts hold what the boundary treatment writes.
 //
-// Every kernel runs one thread per interior cell, r fastest.  The cell
+// The kernels of a step take the cells in runs along x, one per thread, r fastest (March).  The cell
 // geometry (face fluxes beta, face vectors S, volume M) is formed from the
 // mesh's triangle vectors (cell.cuh) and the Q1 velocity in FP64 in the dt and
 // predictor kernels, with the reference's face and volume quadrature sums
-// evaluated in closed form (fv_geometry).
+// evaluated in closed form (FvWalk).
 //
 // The antidiffusive flux of cell i towards neighbour j is F_ij = dt / M_i
 // |beta_ij| / 2 (T_i - T_j): apart from M_i it is the same for both sides of a
@@ -21,7 +21,7 @@
 // and two reads; those and T_L, R+ and R- are what bounds the step).  A cell takes
 // its upper faces from its upper neighbours' entries; the last cell in a direction
 // stores its own upper face in the ghost cell there.  Level 7 (20,971,520 cells):
-// step 2.09 -> 1.39 ms, stable dt 0.81 -> 0.53 ms.
+// step 2.09 -> 1.20 ms, stable dt 0.81 -> 0.46 ms.
 #include <algorithm>
 
 #include "cell.cuh"
@@ -49,10 +49,10 @@ struct FvGeom
     const double*        radii;
     Ptr3< const double > cen; // FV cell centres with ghosts
     Ptr3< const double > vel; // Q1 velocity (stored nodes)
-    const uint8_t*       orient; // face orientation bits per cell (nullptr: the centre test)
+    const uint8_t*       orient; // face orientation bits per cell
 };
 
-// GeometryHelper::compute_geometry (geometry_helper.hpp:180-363) in closed form.
+// GeometryHelper::compute_geometry (geometry_helper.hpp:180-363) in closed form (the sums are FvWalk's, below).
 //
 // The reference integrates each face of the two wedges of the cell with a
 // quadrature rule over the wedge map x = r(zeta) (p0 + xi a + eta b),
@@ -76,98 +76,40 @@ struct FvGeom
 //     are tabulated (iM = 1 / M, fv_inverse_volume).
 // These are the same sums (exact algebra, different rounding: ~1e-16
 // relative), about 120 FP64 operations per cell instead of ~3,000, with b x p0,
-// a x p0 = -(p0 x a), a x b and 1 / ((a x b) . p0) from the triangle table.  Every
-// face is then oriented from this cell towards the neighbour's centre.
-// WITH_VELOCITY: the face fluxes beta (false: geometry only); WITH_S: the face vectors S, needed by the
-// orientation test and the diffusion term only (with the orientation bits and no diffusivity they are dead).
-template < bool WITH_VELOCITY = true, bool WITH_S = true >
-__device__ void fv_geometry( const FvGeom& G, int d, int x, int y, int r, double beta[6], double& iM, double S[6][3],
-                             uint8_t* flips = nullptr )
+// a x p0 = -(p0 x a), a x b and 1 / ((a x b) . p0) from the triangle table (FvWalk).  Every
+// face is oriented from its cell towards the neighbour's centre: that test, here, is
+// made once per mesh and kept as one bit per face (set: the normal points inwards).
+__device__ __forceinline__ unsigned inward_faces( const FvGeom& G, int d, int x, int y, int r )
 {
     const int    N = G.N, n1 = N + 1, n2 = N + 2;
     const double r1 = G.radii[d * n1 + r - 1], r2 = G.radii[d * n1 + r];
-    const double g  = 0.5773502691896258; // 1 / sqrt(3)
-    const double h  = 0.5 * ( r2 - r1 );
-    const double rm = r1 + h * ( 1.0 - g ), rp = r1 + h * ( 1.0 + g ); // r(-g), r(+g)
-    const double Rb = 0.25 * ( rm * ( 1.0 + g ) + rp * ( 1.0 - g ) ), Rt = 0.25 * ( rm * ( 1.0 - g ) + rp * ( 1.0 + g ) );
-    const double rs = rm + rp, r1s = r1 * r1, r2s = r2 * r2;
-#pragma unroll
-    for ( int n = 0; n < 6; ++n )
-    {
-        beta[n] = 0.0;
-        S[n][0] = S[n][1] = S[n][2] = 0.0;
-    }
-    unsigned node[4];
-    cell_nodes( n1, d, x - 1, y - 1, r - 1, node );
-#pragma unroll
-    for ( int w = 0; w < 2; ++w )
-    {
-        const Triangle< double > t( G.table, N, d, x - 1, y - 1, w );
-        double                   u[6][3];
-#pragma unroll
-        for ( int i = 0; i < 6; ++i )
-        {
-            const unsigned id = node[wedge_node( w, i, 0 ) + 2 * wedge_node( w, i, 1 )] + i / 3;
-#pragma unroll
-            for ( int c = 0; c < 3; ++c )
-                u[i][c] = WITH_VELOCITY ? G.vel.p[c][id] : 0.0;
-        }
-        const double *ab = t.v, *bp = t.b1, ap[3] = { -t.b2[0], -t.b2[1], -t.b2[2] };
-        const int nx = w == 0 ? 0 : 1, ny = w == 0 ? 2 : 3; // the wedge's xi = 0 and eta = 0 faces
-        double    bx = 0.0, by = 0.0, bl = 0.0, bt = 0.0;
-#pragma unroll
-        for ( int c = 0; c < 3; ++c )
-        {
-            bx += bp[c] * ( Rb * ( u[0][c] + u[2][c] ) + Rt * ( u[3][c] + u[5][c] ) );
-            by += ap[c] * ( Rb * ( u[0][c] + u[1][c] ) + Rt * ( u[3][c] + u[4][c] ) );
-            bl += ab[c] * ( u[0][c] + u[1][c] + u[2][c] );
-            bt += ab[c] * ( u[3][c] + u[4][c] + u[5][c] );
-            if ( WITH_S )
-            {
-                S[nx][c] += rs * h * bp[c];
-                S[ny][c] += rs * h * ap[c];
-                S[4][c] += 0.5 * r1s * ab[c];
-                S[5][c] += 0.5 * r2s * ab[c];
-            }
-        }
-        beta[nx] += h * bx;
-        beta[ny] += h * by;
-        beta[4] += r1s / 6.0 * bl;
-        beta[5] += r2s / 6.0 * bt;
-    }
-    iM = fv_inverse_volume( G.table, N, d, x - 1, y - 1, r - 1 );
-    // orient every face from this cell towards the neighbour's centre: from the mesh's orientation bits (the
-    // same test, made once per mesh), else the test itself
+    const double g = 0.5773502691896258, h = 0.5 * ( r2 - r1 ); // g = 1 / sqrt(3)
+    const double rs = ( r1 + h * ( 1.0 - g ) ) + ( r1 + h * ( 1.0 + g ) );
+    const Triangle< double > t0( G.table, N, d, x - 1, y - 1, 0 ), t1( G.table, N, d, x - 1, y - 1, 1 );
     const size_t ci   = fv_index( n2, d, x, y, r );
     unsigned     bits = 0;
-    if ( G.orient )
-        bits = G.orient[ci];
-    else if ( WITH_S )
+    double       dc[6] = { 0.0, 0.0, 0.0, 0.0, 0.0, 0.0 };
+#pragma unroll
+    for ( int c = 0; c < 3; ++c )
     {
+        const double S[6] = { rs * h * t0.b1[c],
+                              rs * h * t1.b1[c],
+                              -rs * h * t0.b2[c],
+                              -rs * h * t1.b2[c],
+                              0.5 * r1 * r1 * ( t0.v[c] + t1.v[c] ),
+                              0.5 * r2 * r2 * ( t0.v[c] + t1.v[c] ) };
 #pragma unroll
-        for ( int nb = 0; nb < 6; ++nb )
+        for ( int n = 0; n < 6; ++n )
         {
-            const size_t cj = fv_index( n2, d, x + kFvOff[nb][0], y + kFvOff[nb][1], r + kFvOff[nb][2] );
-            double       dc = 0.0;
-#pragma unroll
-            for ( int a = 0; a < 3; ++a )
-                dc += S[nb][a] * ( G.cen.p[a][cj] - G.cen.p[a][ci] );
-            if ( dc < 0 )
-                bits |= 1u << nb;
+            const size_t cj = fv_index( n2, d, x + kFvOff[n][0], y + kFvOff[n][1], r + kFvOff[n][2] );
+            dc[n] += S[n] * ( G.cen.p[c][cj] - G.cen.p[c][ci] );
         }
     }
-    if ( flips )
-        *flips = uint8_t( bits );
 #pragma unroll
-    for ( int nb = 0; nb < 6; ++nb )
-        if ( bits >> nb & 1u )
-        {
-            if ( WITH_S )
-#pragma unroll
-                for ( int a = 0; a < 3; ++a )
-                    S[nb][a] = -S[nb][a];
-            beta[nb] = -beta[nb];
-        }
+    for ( int n = 0; n < 6; ++n )
+        if ( dc[n] < 0 )
+            bits |= 1u << n;
+    return bits;
 }
 
 __device__ __forceinline__ bool cell_of_thread( int N, int& d, int& x, int& y, int& r )
@@ -236,52 +178,198 @@ __global__ void fv_ghost_kernel( int N, const int* __restrict__ map, Ptr3< doubl
 
 // compute_dt_stable (fct_advection_diffusion.hpp:193-254): min over cells of
 // M / (inflow + diffusion); positive doubles order like their bit patterns
-// the face orientation bits of every interior cell (fv_geometry's centre test, no velocity)
+// the face orientation bits of every interior cell (the centre test of inward_faces)
 __global__ void __launch_bounds__( kFvThreads ) orient_kernel( FvGeom G, uint8_t* bits )
 {
     int d, x, y, r;
     if ( !cell_of_thread( G.N, d, x, y, r ) )
         return;
-    double beta[6], iM, S[6][3];
-    fv_geometry< false >( G, d, x, y, r, beta, iM, S, bits + fv_index( G.N + 2, d, x, y, r ) );
+    bits[fv_index( G.N + 2, d, x, y, r )] = uint8_t( inward_faces( G, d, x, y, r ) );
 }
 
-// Blocks take the cells in turn and one atomic per block closes the minimum: one per warp on the single result cost
+// The geometry and face fluxes of a run of cells in x (the sums above): the velocity at the four nodes of the
+// upper x face and the face's flux and vector stay for the next cell, whose lower x face it is, so a cell after the
+// first loads 12 node values instead of 24 and forms 7 of the 8 wedge faces.
+template < bool DIFFUSION >
+struct FvWalk
+{
+    double h, hb, ht, b6, t6, rs, b2, t2; // h; h R_b, h R_t, r1^2 / 6, r2^2 / 6; h (r(-g) + r(g)), r1^2 / 2, r2^2 / 2
+    double u[2][2][3];                    // lower x nodes: [y][bottom, top][component]
+    double face, S[3];                    // upper x face of the cell before, seen from there
+
+    __device__ __forceinline__ void plane( const FvGeom& G, int d, int x, int y, int r, double ( &v )[2][2][3] ) const
+    {
+        const int      n1 = G.N + 1;
+        const unsigned id = unsigned( ( ( d * n1 + x ) * n1 + y ) ) * n1 + r;
+#pragma unroll
+        for ( int c = 0; c < 3; ++c )
+        {
+            const double* const p = G.vel.p[c] + id;
+            v[0][0][c] = p[0], v[0][1][c] = p[1], v[1][0][c] = p[n1], v[1][1][c] = p[n1 + 1];
+        }
+    }
+    // flux and vector of the quad over the nodes a, b with the lateral vector n
+    __device__ __forceinline__ double quad( const double* n, const double ( &a )[2][3], const double ( &b )[2][3], double* s ) const
+    {
+        double f = 0.0;
+#pragma unroll
+        for ( int c = 0; c < 3; ++c )
+        {
+            f += n[c] * ( hb * ( a[0][c] + b[0][c] ) + ht * ( a[1][c] + b[1][c] ) );
+            if ( DIFFUSION )
+                s[c] = rs * n[c];
+        }
+        return f;
+    }
+    // cell (x, y, r), x the first of the run
+    __device__ __forceinline__ void begin( const FvGeom& G, int d, int x, int y, int r )
+    {
+        const double r1 = G.radii[d * ( G.N + 1 ) + r - 1], r2 = G.radii[d * ( G.N + 1 ) + r], g = 0.5773502691896258;
+        h = 0.5 * ( r2 - r1 );
+        const double rm = r1 + h * ( 1.0 - g ), rp = r1 + h * ( 1.0 + g );
+        hb = h * ( 0.25 * ( rm * ( 1.0 + g ) + rp * ( 1.0 - g ) ) ), ht = h * ( 0.25 * ( rm * ( 1.0 - g ) + rp * ( 1.0 + g ) ) );
+        rs = h * ( rm + rp ), b6 = r1 * r1 / 6.0, t6 = r2 * r2 / 6.0, b2 = 0.5 * r1 * r1, t2 = 0.5 * r2 * r2;
+        plane( G, d, x - 1, y - 1, r - 1, u );
+        const Triangle< double > t( G.table, G.N, d, x - 1, y - 1, 0 );
+        face = quad( t.b1, u[0], u[1], S );
+        if ( G.orient[fv_index( G.N + 2, d, x, y, r )] & 1u )
+            turn( face, S );
+        turn( face, S ); // as the cell before would see it
+    }
+    __device__ __forceinline__ static void turn( double& f, double* s )
+    {
+        f = -f;
+        if ( DIFFUSION )
+#pragma unroll
+            for ( int c = 0; c < 3; ++c )
+                s[c] = -s[c];
+    }
+    __device__ __forceinline__ void cell( const FvGeom& G, int d, int x, int y, int r, double ( &beta )[6], double& iM,
+                                          double ( &Sf )[6][3] )
+    {
+        const unsigned bits = G.orient[fv_index( G.N + 2, d, x, y, r )];
+        double         v[2][2][3];
+        plane( G, d, x, y - 1, r - 1, v );
+        const Triangle< double > t0( G.table, G.N, d, x - 1, y - 1, 0 ), t1( G.table, G.N, d, x - 1, y - 1, 1 );
+        const double             n0[3] = { -t0.b2[0], -t0.b2[1], -t0.b2[2] }, n1[3] = { -t1.b2[0], -t1.b2[1], -t1.b2[2] };
+        beta[0] = face;
+        if ( DIFFUSION )
+#pragma unroll
+            for ( int c = 0; c < 3; ++c )
+                Sf[0][c] = S[c];
+        turn( beta[0], Sf[0] );
+        beta[1] = quad( t1.b1, v[1], v[0], Sf[1] );
+        beta[2] = quad( n0, u[0], v[0], Sf[2] );
+        beta[3] = quad( n1, v[1], u[1], Sf[3] );
+        double f[2][2] = { { 0.0, 0.0 }, { 0.0, 0.0 } };
+#pragma unroll
+        for ( int c = 0; c < 3; ++c )
+        {
+#pragma unroll
+            for ( int k = 0; k < 2; ++k )
+            {
+                const double m = u[1][k][c] + v[0][k][c]; // the edge both wedges share
+                f[k][0] += t0.v[c] * ( u[0][k][c] + m );
+                f[k][1] += t1.v[c] * ( v[1][k][c] + m );
+            }
+            if ( DIFFUSION )
+                Sf[4][c] = b2 * ( t0.v[c] + t1.v[c] ), Sf[5][c] = t2 * ( t0.v[c] + t1.v[c] );
+        }
+        beta[4] = b6 * ( f[0][0] + f[0][1] ), beta[5] = t6 * ( f[1][0] + f[1][1] );
+        iM = fv_inverse_volume( G.table, G.N, d, x - 1, y - 1, r - 1 );
+#pragma unroll
+        for ( int n = 1; n < 6; ++n )
+            if ( bits >> n & 1u )
+                turn( beta[n], Sf[n] );
+        face = beta[1];
+#pragma unroll
+        for ( int c = 0; c < 3; ++c )
+        {
+            if ( DIFFUSION )
+                S[c] = Sf[1][c];
+#pragma unroll
+            for ( int k = 0; k < 2; ++k )
+                u[0][k][c] = v[0][k][c], u[1][k][c] = v[1][k][c];
+        }
+    }
+};
+
+// The kernels of a step march: a thread owns a (y, r) and takes `run` cells in x, so what it reads of the x
+// neighbours (and in FvWalk forms of the shared face) comes from the cell before, and a block holds several y of 32
+// cells in r, so most of the y neighbours come from L1.  With one cell per thread the limiter and the correction
+// read each plane about twice from L2 and were bound by that, and the other two loaded every node and formed every
+// x face twice.  Level 7: limiter 306 -> 255 us, correction 351 -> 270 us, predictor 625 -> 540 us, dt 511 -> 440 us.
+// The run leaves at least 1,024 threads per SM (step at level 5, runs of 1 / 2: 56.4 / 52.2 us; level 6, 2 / 4 / 8:
+// 210 / 198 / 200 us) and gains nothing above 8 cells (level 7, 4 / 8 / 16 in the limiter and the correction: 1,289 /
+// 1,269 / 1,267 us the step).
+struct March
+{
+    int run, lanes, rows; // cells in x per thread; r lanes and y rows of a block
+    unsigned blocks;
+};
+
+March march_shape( const tn_mesh* m )
+{
+    March           s;
+    const long long cells = (long long) kDiamonds * m->N * m->N * m->N;
+    s.run   = int( std::clamp( cells / ( 148LL * 1024 ), 1LL, 8LL ) );
+    s.lanes = std::min( m->N, 32 );
+    s.rows  = kFvThreads / s.lanes;
+    s.blocks = unsigned( kDiamonds * ( ( m->N + s.run - 1 ) / s.run ) ) * unsigned( ( m->N + s.rows - 1 ) / s.rows ) *
+               unsigned( m->N / s.lanes );
+    return s;
+}
+
+// y and r of this thread in block b, its diamond and first x; false: no cell
+__device__ __forceinline__ bool march_of_thread( int N, const March& s, unsigned b, int& d, int& x, int& y, int& r )
+{
+    const unsigned rb = unsigned( N / s.lanes ), yb = unsigned( ( N + s.rows - 1 ) / s.rows ), xb = unsigned( ( N + s.run - 1 ) / s.run );
+    r = int( b % rb ) * s.lanes + int( threadIdx.x ) % s.lanes + 1, b /= rb;
+    y = int( b % yb ) * s.rows + int( threadIdx.x ) / s.lanes + 1, b /= yb;
+    x = int( b % xb ) * s.run + 1, d = int( b / xb );
+    return y <= N;
+}
+
+// Blocks take the runs in turn and one atomic per block closes the minimum: one per warp on the single result cost
 // as much as the geometry (level 7: 655,360 of them).
 template < bool DIFFUSION >
-__global__ void __launch_bounds__( kFvThreads, 4 ) dt_kernel( FvGeom G, double kappa, unsigned long long* out )
+__global__ void __launch_bounds__( kFvThreads, 4 ) dt_kernel( FvGeom G, March s, double kappa, unsigned long long* out )
 {
     __shared__ double sh[kFvThreads / 32];
-    const long long   cells = (long long) kDiamonds * G.N * G.N * G.N;
-    const int         n2    = G.N + 2;
-    double            dtc   = 1e300;
-    for ( long long t = blockIdx.x * (long long) kFvThreads + threadIdx.x; t < cells; t += (long long) gridDim.x * kFvThreads )
+    const int         n2  = G.N + 2;
+    double            dtc = 1e300;
+    for ( unsigned b = blockIdx.x; b < s.blocks; b += gridDim.x )
     {
-        int    d, x, y, r;
-        double beta[6], iM, S[6][3], lambda = 0.0;
-        cell_of( t, G.N, d, x, y, r );
-        ++x, ++y, ++r;
-        fv_geometry< true, DIFFUSION >( G, d, x, y, r, beta, iM, S );
-        const size_t ci = fv_index( n2, d, x, y, r );
-#pragma unroll
-        for ( int n = 0; n < 6; ++n )
+        int d, x, y, r;
+        if ( !march_of_thread( G.N, s, b, d, x, y, r ) )
+            continue;
+        FvWalk< DIFFUSION > walk;
+        walk.begin( G, d, x, y, r );
+        for ( const int end = min( x + s.run, G.N + 1 ); x < end; ++x )
         {
-            if ( beta[n] < 0 )
-                lambda -= beta[n];
-            if ( DIFFUSION && kappa > 0 )
+            double beta[6], iM, S[6][3], lambda = 0.0;
+            walk.cell( G, d, x, y, r, beta, iM, S );
+            const size_t ci = fv_index( n2, d, x, y, r );
+#pragma unroll
+            for ( int n = 0; n < 6; ++n )
             {
-                const size_t cj  = fv_index( n2, d, x + kFvOff[n][0], y + kFvOff[n][1], r + kFvOff[n][2] );
-                double       den = 0.0, ss = 0.0;
-                for ( int a = 0; a < 3; ++a )
+                if ( beta[n] < 0 )
+                    lambda -= beta[n];
+                if ( DIFFUSION && kappa > 0 )
                 {
-                    den += ( G.cen.p[a][cj] - G.cen.p[a][ci] ) * S[n][a];
-                    ss += S[n][a] * S[n][a];
+                    const size_t cj  = fv_index( n2, d, x + kFvOff[n][0], y + kFvOff[n][1], r + kFvOff[n][2] );
+                    double       den = 0.0, ss = 0.0;
+                    for ( int a = 0; a < 3; ++a )
+                    {
+                        den += ( G.cen.p[a][cj] - G.cen.p[a][ci] ) * S[n][a];
+                        ss += S[n][a] * S[n][a];
+                    }
+                    if ( den > 0 )
+                        lambda += kappa * ss / den;
                 }
-                if ( den > 0 )
-                    lambda += kappa * ss / den;
             }
+            dtc = fmin( dtc, lambda > 0 ? 1.0 / ( iM * lambda ) : 1e30 );
         }
-        dtc = fmin( dtc, lambda > 0 ? 1.0 / ( iM * lambda ) : 1e30 );
     }
     for ( int off = 16; off > 0; off >>= 1 )
         dtc = fmin( dtc, __shfl_down_sync( 0xffffffffu, dtc, off ) );
@@ -296,56 +384,63 @@ __global__ void __launch_bounds__( kFvThreads, 4 ) dt_kernel( FvGeom G, double k
     }
 }
 
-// FCTPredictorKernel (fct_advection_diffusion.hpp:262-376); DIFFUSION: kappa != 0
+// FCTPredictorKernel (fct_advection_diffusion.hpp:262-376); DIFFUSION: kappa != 0 (with 4 blocks per SM its spills cost
+// more than the occupancy gives: level 7 step 1,765 -> 1,809 us; 5 blocks without it: 1,196 -> 1,241 us)
 template < bool DIFFUSION >
-__global__ void __launch_bounds__( kFvThreads, DIFFUSION ? 4 : 6 )
-    predictor_kernel( FvGeom G, const double* __restrict__ T, double* __restrict__ TL, double* __restrict__ g, double dt,
-                      double kappa, const double* __restrict__ src, int subtract_divergence )
+__global__ void __launch_bounds__( kFvThreads, DIFFUSION ? 3 : 4 )
+    predictor_kernel( FvGeom G, March s, const double* __restrict__ T, double* __restrict__ TL, double* __restrict__ g,
+                      double dt, double kappa, const double* __restrict__ src, int subtract_divergence )
 {
     int d, x, y, r;
-    if ( !cell_of_thread( G.N, d, x, y, r ) )
+    if ( !march_of_thread( G.N, s, blockIdx.x, d, x, y, r ) )
         return;
-    const int n2 = G.N + 2;
-    double    beta[6], iM, S[6][3];
-    fv_geometry< true, DIFFUSION >( G, d, x, y, r, beta, iM, S );
-    const size_t i  = fv_index( n2, d, x, y, r );
-    const size_t nf = size_t( kDiamonds ) * n2 * n2 * n2; // g holds 3 planes of nf (SoA)
-    const double Ti = T[i];
-    double       lo_diag = 0.0, lo_update = 0.0, bsum = 0.0;
-#pragma unroll
-    for ( int n = 0; n < 6; ++n )
+    const int           n2 = G.N + 2, sx = n2 * n2, end = min( x + s.run, G.N + 1 );
+    const size_t        nf = size_t( kDiamonds ) * n2 * sx; // g holds 3 planes of nf (SoA)
+    size_t              i  = fv_index( n2, d, x, y, r );
+    double              below = T[i - sx], Ti = T[i];
+    FvWalk< DIFFUSION > walk;
+    walk.begin( G, d, x, y, r );
+    for ( ; x < end; ++x, i += sx )
     {
-        const size_t j  = fv_index( n2, d, x + kFvOff[n][0], y + kFvOff[n][1], r + kFvOff[n][2] );
-        const double Tj = T[j];
-        if ( beta[n] >= 0 )
-            lo_diag += beta[n];
-        else
-            lo_update += beta[n] * Tj;
-        bsum += beta[n];
-        if ( DIFFUSION ) // the diffusion term; zero without diffusivity (no centre loads)
+        const double above = T[i + sx], Tn[6] = { below, above, T[i - n2], T[i + n2], T[i - 1], T[i + 1] };
+        double       beta[6], iM, S[6][3], lo_diag = 0.0, lo_update = 0.0, bsum = 0.0;
+        walk.cell( G, d, x, y, r, beta, iM, S );
+#pragma unroll
+        for ( int n = 0; n < 6; ++n )
         {
-            double den = 0.0, ss = 0.0;
-            for ( int a = 0; a < 3; ++a )
+            const size_t j  = n / 2 == 0 ? ( n % 2 ? i + sx : i - sx ) : ( n / 2 == 1 ? ( n % 2 ? i + n2 : i - n2 ) : ( n % 2 ? i + 1 : i - 1 ) );
+            const double Tj = Tn[n];
+            if ( beta[n] >= 0 )
+                lo_diag += beta[n];
+            else
+                lo_update += beta[n] * Tj;
+            bsum += beta[n];
+            if ( DIFFUSION ) // the diffusion term; zero without diffusivity (no centre loads)
             {
-                den += ( G.cen.p[a][j] - G.cen.p[a][i] ) * S[n][a];
-                ss += S[n][a] * S[n][a];
+                double den = 0.0, ss = 0.0;
+                for ( int a = 0; a < 3; ++a )
+                {
+                    den += ( G.cen.p[a][j] - G.cen.p[a][i] ) * S[n][a];
+                    ss += S[n][a] * S[n][a];
+                }
+                const double dc = kappa * ( ss / den );
+                lo_diag += dc;
+                lo_update -= dc * Tj;
             }
-            const double dc = kappa * ( ss / den );
-            lo_diag += dc;
-            lo_update -= dc * Tj;
+            // face 2a towards the lower neighbour in direction a; the last cell's upper face goes to the ghost cell
+            if ( n % 2 == 0 )
+                g[( n / 2 ) * nf + i] = fabs( beta[n] ) * 0.5 * ( Ti - Tj );
+            else if ( ( n == 1 ? x : ( n == 3 ? y : r ) ) == G.N )
+                g[( n / 2 ) * nf + j] = fabs( beta[n] ) * 0.5 * ( Tj - Ti );
         }
-        // face 2a towards the lower neighbour in direction a; the last cell's upper face goes to the ghost cell
-        if ( n % 2 == 0 )
-            g[( n / 2 ) * nf + i] = fabs( beta[n] ) * 0.5 * ( Ti - Tj );
-        else if ( ( n == 1 ? x : ( n == 3 ? y : r ) ) == G.N )
-            g[( n / 2 ) * nf + j] = fabs( beta[n] ) * 0.5 * ( Tj - Ti );
+        if ( subtract_divergence )
+            lo_diag -= bsum;
+        double tl = Ti - ( dt * iM ) * ( lo_diag * Ti + lo_update );
+        if ( src )
+            tl += dt * src[i];
+        TL[i] = tl;
+        below = Ti, Ti = above;
     }
-    if ( subtract_divergence )
-        lo_diag -= bsum;
-    double tl = Ti - ( dt * iM ) * ( lo_diag * Ti + lo_update );
-    if ( src )
-        tl += dt * src[i];
-    TL[i] = tl;
 }
 
 // apply_dirichlet_bcs (fv/hex/helpers.hpp:26-64): thread per lateral column
@@ -362,67 +457,70 @@ __global__ void dirichlet_kernel( int N, double* __restrict__ T, double t_cmb, d
         T[fv_index( n2, d, x, y, N )] = T[fv_index( n2, d, x, y, N + 1 )] = t_surf;
 }
 
-// the six antidiffusive fluxes of cell i (dt / M_i times its faces' g)
-__device__ __forceinline__ void antidiffusive( const double* __restrict__ g, size_t nf, int n2, size_t i, double scale, double f[6] )
-{
-    const size_t step[3] = { size_t( n2 ) * n2, size_t( n2 ), 1 };
-#pragma unroll
-    for ( int a = 0; a < 3; ++a )
-    {
-        f[2 * a]     = scale * g[a * nf + i];
-        f[2 * a + 1] = -scale * g[a * nf + i + step[a]];
-    }
-}
-
-// FCTLimiterKernel (fct_advection_diffusion.hpp:486-531)
+// FCTLimiterKernel (fct_advection_diffusion.hpp:486-531); the six antidiffusive fluxes of a cell are dt / M times its
+// faces' g
 __global__ void __launch_bounds__( kFvThreads )
-    limiter_kernel( FvGeom G, const double* __restrict__ TL, const double* __restrict__ g, double dt, double* __restrict__ Rp,
-                    double* __restrict__ Rm )
+    limiter_kernel( FvGeom G, March s, const double* __restrict__ TL, const double* __restrict__ g, double dt,
+                    double* __restrict__ Rp, double* __restrict__ Rm )
 {
     int d, x, y, r;
-    if ( !cell_of_thread( G.N, d, x, y, r ) )
+    if ( !march_of_thread( G.N, s, blockIdx.x, d, x, y, r ) )
         return;
-    const int    n2 = G.N + 2;
-    const size_t i  = fv_index( n2, d, x, y, r );
-    const double ti = TL[i];
-    double       f[6], Pp = 0.0, Pm = 0.0, tmax = ti, tmin = ti;
-    antidiffusive( g, size_t( kDiamonds ) * n2 * n2 * n2, n2, i, dt * fv_inverse_volume( G.table, G.N, d, x - 1, y - 1, r - 1 ), f );
-#pragma unroll
-    for ( int n = 0; n < 6; ++n )
+    const int    n2 = G.N + 2, sx = n2 * n2, end = min( x + s.run, G.N + 1 );
+    const size_t nf = size_t( kDiamonds ) * n2 * sx;
+    size_t       i  = fv_index( n2, d, x, y, r );
+    double       below = TL[i - sx], ti = TL[i], gx = g[i];
+    for ( ; x < end; ++x, i += sx )
     {
-        if ( f[n] > 0 )
-            Pp += f[n];
-        else
-            Pm += f[n];
-        const double tj = TL[fv_index( n2, d, x + kFvOff[n][0], y + kFvOff[n][1], r + kFvOff[n][2] )];
-        tmax            = fmax( tmax, tj );
-        tmin            = fmin( tmin, tj );
+        const double* const gy = g + nf + i;
+        const double* const gr = gy + nf;
+        const double        above = TL[i + sx], gu = g[i + sx];
+        const double        tn[4] = { TL[i - n2], TL[i + n2], TL[i - 1], TL[i + 1] };
+        const double        scale = dt * fv_inverse_volume( G.table, G.N, d, x - 1, y - 1, r - 1 );
+        const double        f[6] = { scale * gx, -scale * gu, scale * gy[0], -scale * gy[n2], scale * gr[0], -scale * gr[1] };
+        double              Pp = 0.0, Pm = 0.0;
+#pragma unroll
+        for ( int n = 0; n < 6; ++n )
+            if ( f[n] > 0 )
+                Pp += f[n];
+            else
+                Pm += f[n];
+        const double tmax = fmax( fmax( fmax( fmax( fmax( fmax( ti, below ), above ), tn[0] ), tn[1] ), tn[2] ), tn[3] );
+        const double tmin = fmin( fmin( fmin( fmin( fmin( fmin( ti, below ), above ), tn[0] ), tn[1] ), tn[2] ), tn[3] );
+        Rp[i] = Pp > 0 ? fmin( 1.0, ( tmax - ti ) / Pp ) : 1.0;
+        Rm[i] = Pm < 0 ? fmin( 1.0, ( tmin - ti ) / Pm ) : 1.0;
+        below = ti, ti = above, gx = gu;
     }
-    Rp[i] = Pp > 0 ? fmin( 1.0, ( tmax - ti ) / Pp ) : 1.0;
-    Rm[i] = Pm < 0 ? fmin( 1.0, ( tmin - ti ) / Pm ) : 1.0;
 }
 
 // FCTCorrectionKernel (fct_advection_diffusion.hpp:605-650)
 __global__ void __launch_bounds__( kFvThreads )
-    correction_kernel( FvGeom G, const double* __restrict__ TL, const double* __restrict__ g, double dt,
+    correction_kernel( FvGeom G, March s, const double* __restrict__ TL, const double* __restrict__ g, double dt,
                        const double* __restrict__ Rp, const double* __restrict__ Rm, double* __restrict__ T )
 {
     int d, x, y, r;
-    if ( !cell_of_thread( G.N, d, x, y, r ) )
+    if ( !march_of_thread( G.N, s, blockIdx.x, d, x, y, r ) )
         return;
-    const int    n2 = G.N + 2;
-    const size_t i  = fv_index( n2, d, x, y, r );
-    const double rp = Rp[i], rm = Rm[i];
-    double       f[6], corr = 0.0;
-    antidiffusive( g, size_t( kDiamonds ) * n2 * n2 * n2, n2, i, dt * fv_inverse_volume( G.table, G.N, d, x - 1, y - 1, r - 1 ), f );
-#pragma unroll
-    for ( int n = 0; n < 6; ++n )
+    const int    n2 = G.N + 2, sx = n2 * n2, end = min( x + s.run, G.N + 1 );
+    const size_t nf = size_t( kDiamonds ) * n2 * sx;
+    size_t       i  = fv_index( n2, d, x, y, r );
+    double       gx = g[i], pb = Rp[i - sx], mb = Rm[i - sx], rp = Rp[i], rm = Rm[i];
+    for ( ; x < end; ++x, i += sx )
     {
-        const size_t j  = fv_index( n2, d, x + kFvOff[n][0], y + kFvOff[n][1], r + kFvOff[n][2] );
-        const double al = f[n] > 0 ? fmin( rp, Rm[j] ) : fmin( rm, Rp[j] );
-        corr += al * f[n];
+        const double* const gy = g + nf + i;
+        const double* const gr = gy + nf;
+        const double        gu = g[i + sx], pa = Rp[i + sx], ma = Rm[i + sx];
+        const double        scale = dt * fv_inverse_volume( G.table, G.N, d, x - 1, y - 1, r - 1 );
+        const double        f[6] = { scale * gx, -scale * gu, scale * gy[0], -scale * gy[n2], scale * gr[0], -scale * gr[1] };
+        const size_t        j[4] = { i - n2, i + n2, i - 1, i + 1 };
+        double              corr = ( f[0] > 0 ? fmin( rp, mb ) : fmin( rm, pb ) ) * f[0];
+        corr += ( f[1] > 0 ? fmin( rp, ma ) : fmin( rm, pa ) ) * f[1];
+#pragma unroll
+        for ( int n = 0; n < 4; ++n )
+            corr += ( f[2 + n] > 0 ? fmin( rp, Rm[j[n]] ) : fmin( rm, Rp[j[n]] ) ) * f[2 + n];
+        T[i] = TL[i] + corr;
+        pb = rp, mb = rm, rp = pa, rm = ma, gx = gu;
     }
-    T[i] = TL[i] + corr;
 }
 
 // Zeroes the ghost cells (all those outside 1..N in some direction) of nf fields: the first and last cell of every
@@ -595,11 +693,12 @@ extern "C" int tn_fct_dt_stable_f64( const tn_mesh* m, const double* const* vel,
     unsigned long long* slot = reinterpret_cast< unsigned long long* >( m->d_red_result + 12 );
     // bytes 0x7f: 1.4e306, above every candidate
     TN_CUDA_TRY( cudaMemsetAsync( slot, 0x7f, sizeof( double ), st ) );
-    const unsigned blocks = std::min( cell_blocks( m ), 148u * 16u );
+    const March    march  = march_shape( m );
+    const unsigned blocks = std::min( march.blocks, 148u * 16u );
     if ( diffusivity != 0.0 )
-        dt_kernel< true ><<< blocks, kFvThreads, 0, st >>>( G, diffusivity, slot );
+        dt_kernel< true ><<< blocks, kFvThreads, 0, st >>>( G, march, diffusivity, slot );
     else
-        dt_kernel< false ><<< blocks, kFvThreads, 0, st >>>( G, diffusivity, slot );
+        dt_kernel< false ><<< blocks, kFvThreads, 0, st >>>( G, march, diffusivity, slot );
     TN_LAUNCH_CHECK();
     TN_CUDA_TRY( cudaMemcpyAsync( dt_stable, slot, sizeof( double ), cudaMemcpyDeviceToHost, st ) );
     TN_CUDA_TRY( cudaStreamSynchronize( st ) );
@@ -636,23 +735,24 @@ extern "C" int tn_fct_step_f64( const tn_mesh* m, double* T, const double* const
     // predictor (fct_advection_diffusion.hpp:384-433) on T with fresh lateral ghosts
     if ( ( rc = ghost_update( m, T, st ) ) )
         return rc;
+    const March march = march_shape( m );
     if ( diffusivity != 0.0 )
-        predictor_kernel< true ><<< cell_blocks( m ), kFvThreads, 0, st >>>( G, T, TL, g, dt, diffusivity, source,
-                                                                             subtract_divergence );
+        predictor_kernel< true ><<< march.blocks, kFvThreads, 0, st >>>( G, march, T, TL, g, dt, diffusivity, source,
+                                                                         subtract_divergence );
     else
-        predictor_kernel< false ><<< cell_blocks( m ), kFvThreads, 0, st >>>( G, T, TL, g, dt, diffusivity, source,
-                                                                              subtract_divergence );
+        predictor_kernel< false ><<< march.blocks, kFvThreads, 0, st >>>( G, march, T, TL, g, dt, diffusivity, source,
+                                                                          subtract_divergence );
     TN_LAUNCH_CHECK();
     if ( bcs && ( rc = tn_fct_apply_dirichlet_f64( m, TL, bcs, s ) ) )
         return rc;
     // limiter (:539-566) and correction (:658-680)
     if ( ( rc = ghost_update( m, TL, st ) ) )
         return rc;
-    limiter_kernel<<< cell_blocks( m ), kFvThreads, 0, st >>>( G, TL, g, dt, Rp, Rm );
+    limiter_kernel<<< march.blocks, kFvThreads, 0, st >>>( G, march, TL, g, dt, Rp, Rm );
     TN_LAUNCH_CHECK();
     if ( ( rc = ghost_update( m, Rp, st, Rm ) ) )
         return rc;
-    correction_kernel<<< cell_blocks( m ), kFvThreads, 0, st >>>( G, TL, g, dt, Rp, Rm, T );
+    correction_kernel<<< march.blocks, kFvThreads, 0, st >>>( G, march, TL, g, dt, Rp, Rm, T );
     TN_LAUNCH_CHECK();
     return TN_OK;
 }

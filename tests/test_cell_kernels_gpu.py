@@ -126,3 +126,23 @@ def test_cg_iterates(case, its):
     r0 = rhs - om.kmass(ones, want, 0)
     dx, m = pcg(lambda v: om.kmass(ones, v, 0), om.dot, r0, its, 1e-12, 1e-12)
     assert abs(n - m) <= 1 and rel(vx.numpy()[0], want + dx) <= 1e-11
+
+
+@pytest.mark.parametrize("L,kappa", [(1, 1e-2), (3, 1e-2), (5, 0.0), (5, 1e-2), (6, 1e-2)])
+def test_fct_runs(L, kappa):
+    """the FCT kernels' runs along x: one cell per thread (1, 3), two (5) and eight (6), fewer than 32 cells in r (1, 3)"""
+    from terraneo_b200 import shell
+    om, pm = Mesh(L), shell.ShellMesh(L)
+    N, rng = om.N, np.random.default_rng(L)
+    vel, c = random_vector(om, seed=L), om.fv_cell_centers()
+    inner = (slice(None),) + (slice(1, N + 1),) * 3
+    T = np.zeros(om.fv_shape)
+    T[inner] = rng.uniform(size=T[inner].shape)
+    fct, v = shell.FCTAdvectionDiffusion(pm), shell.VectorQ1Vec(pm)
+    v.set_numpy(vel)
+    dt = om.fct_dt_stable(c, vel, kappa)
+    assert fct.dt_stable(v, kappa) == pytest.approx(dt, rel=1e-12)
+    ref, _ = om.fct_step(c, vel, om.fv_ghost_update(T), 0.5 * dt, kappa, None, True, None)
+    Tg = torch.as_tensor(T, device="cuda")
+    fct.step(Tg, v, 0.5 * dt, kappa, None, True, None)
+    assert rel(Tg.cpu().numpy()[inner], ref[inner]) <= 1e-12  # the tolerance of the level-2 and 4 tests times ten: rough fields
