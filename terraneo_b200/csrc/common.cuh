@@ -115,6 +115,7 @@ struct tn_mesh
     std::vector< double > h_radii;     // [nd][n1]
     std::vector< uint8_t > h_lat_owned; // [nd][n1][n1]
 
+    char*    d_block    = nullptr; // the one allocation of the arrays formed with the mesh (mesh_create_diamonds)
     double*  d_coords   = nullptr;
     double*  d_radii    = nullptr;
     float*   d_coords32 = nullptr;
@@ -139,7 +140,7 @@ struct tn_mesh
     uint8_t* d_fv_orient = nullptr;
 
     tn_lateral_tables laplace_tables, mass_tables;
-    // wedge vectors per triangle (cell.cuh), one allocation
+    // wedge vectors per triangle (cell.cuh)
     double* d_triangles   = nullptr;
     float*  d_triangles32 = nullptr;
 

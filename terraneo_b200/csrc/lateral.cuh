@@ -522,6 +522,20 @@ T*& lateral_slot( double*& d, float*& f )
         return f;
 }
 
+// values of an operator's stencil and radial tables on mesh m, and the launch that fills them
+template < typename OP >
+size_t lateral_table_words( const tn_mesh* m, bool radial )
+{
+    return radial ? size_t( OP::R ) * m->N : size_t( kStencil * OP::K ) * m->nlat;
+}
+template < typename OP, typename T >
+bool lateral_fill( const tn_mesh* m, T* lat, T* rad, cudaStream_t st )
+{
+    const size_t n = std::max( m->nlat, size_t( m->N ) );
+    lateral_table_kernel< OP, T ><<< unsigned( ( n + 127 ) / 128 ), 128, 0, st >>>( m->N, m->nlat, m->d_coords, m->d_radii, lat, rad );
+    return cudaGetLastError() == cudaSuccess;
+}
+
 // An operator's tables in the precision of T, built on the mesh's first use of them and complete for every stream
 // when this returns; false when that fails.
 template < typename OP, typename T >
@@ -533,16 +547,15 @@ bool lateral_tables( const tn_mesh* m, tn_lateral_tables tn_mesh::*which, Latera
     T *&                          dlat = lateral_slot< T >( t.lat, t.lat32 ), *&drad = lateral_slot< T >( t.rad, t.rad32 );
     if ( !dlat )
     {
-        const size_t nl = size_t( kStencil * OP::K ) * m->nlat, n = std::max( m->nlat, size_t( m->N ) );
-        T *          l = nullptr, *r = nullptr;
-        if ( cudaMalloc( &l, nl * sizeof( T ) ) != cudaSuccess || cudaMalloc( &r, size_t( OP::R ) * m->N * sizeof( T ) ) != cudaSuccess )
+        T *l = nullptr, *r = nullptr;
+        if ( cudaMalloc( &l, lateral_table_words< OP >( m, false ) * sizeof( T ) ) != cudaSuccess ||
+             cudaMalloc( &r, lateral_table_words< OP >( m, true ) * sizeof( T ) ) != cudaSuccess )
         {
             (void) cudaGetLastError();
             cudaFree( l );
             return false;
         }
-        lateral_table_kernel< OP, T ><<< unsigned( ( n + 127 ) / 128 ), 128, 0, st >>>( m->N, m->nlat, m->d_coords, m->d_radii, l, r );
-        if ( cudaGetLastError() != cudaSuccess || cudaStreamSynchronize( st ) != cudaSuccess )
+        if ( !lateral_fill< OP, T >( m, l, r, st ) || cudaStreamSynchronize( st ) != cudaSuccess )
         {
             (void) cudaGetLastError();
             cudaFree( l );

@@ -169,17 +169,14 @@ int kmass_apply( const tn_mesh* m, const T* k, int mode, int apply_mode, int com
     return TN_OK;
 }
 
-// The stencils of the plain mass matrix, both precisions, with the mesh: its apply had no table before it was
-// separated, so a first one may not allocate or wait (it may be inside a stream capture).
-int build_mass_tables( tn_mesh* m )
+// The stencils of the plain mass matrix are formed with the mesh, in both precisions: its apply had no table before it
+// was separated, so a first one may not allocate or wait (it may be inside a stream capture).
+size_t mass_table_words( const tn_mesh* m, bool radial ) { return lateral_table_words< MassOp< double > >( m, radial ); }
+bool   fill_mass_tables( const tn_mesh* m )
 {
-    LateralParams< double > P{};
-    LateralParams< float >  Q{};
-    if ( lateral_tables< MassOp< double > >( m, &tn_mesh::mass_tables, P, nullptr ) &&
-         lateral_tables< MassOp< float > >( m, &tn_mesh::mass_tables, Q, nullptr ) )
-        return TN_OK;
-    set_error( "tn_mesh_create: allocating the lateral stencils of the mass matrix failed" );
-    return TN_ERR_NOMEM;
+    const tn_lateral_tables& t = m->mass_tables;
+    return lateral_fill< MassOp< double >, double >( m, t.lat, t.rad, nullptr ) &&
+           lateral_fill< MassOp< float >, float >( m, t.lat32, t.rad32, nullptr );
 }
 
 // CG on the plain mass matrix from x's values (lateral_cg.cuh); fields: 4 stored-node fields

@@ -99,15 +99,39 @@ void diamond_lateral_points( int diamond, int N, double* out /* [n1][n1][3] */ )
     }
 }
 
-// a device copy of n host values (an empty array still gets a one-element allocation)
-template < typename T >
-int upload( const T* h, size_t n, T** d )
+// The device arrays of a mesh in one allocation: placed first, then allocated together and filled from the host arrays
+// named.
+class MeshArrays
 {
-    TN_CUDA_TRY( cudaMalloc( d, std::max< size_t >( n, 1 ) * sizeof( T ) ) );
-    if ( n )
-        TN_CUDA_TRY( cudaMemcpy( *d, h, n * sizeof( T ), cudaMemcpyHostToDevice ) );
-    return TN_OK;
-}
+  public:
+    template < typename T >
+    void place( T*& p, size_t n, const T* from = nullptr )
+    {
+        items_.push_back( { reinterpret_cast< void** >( &p ), from, n * sizeof( T ), bytes_ } );
+        bytes_ += ( std::max< size_t >( n, 1 ) * sizeof( T ) + 255 ) / 256 * 256;
+    }
+    int allocate( char** block ) const
+    {
+        TN_CUDA_TRY( cudaMalloc( block, bytes_ ) );
+        for ( const Item& i : items_ )
+        {
+            *i.p = *block + i.offset;
+            if ( i.from && i.bytes )
+                TN_CUDA_TRY( cudaMemcpy( *i.p, i.from, i.bytes, cudaMemcpyHostToDevice ) );
+        }
+        return TN_OK;
+    }
+
+  private:
+    struct Item
+    {
+        void**      p;
+        const void* from;
+        size_t      bytes, offset;
+    };
+    std::vector< Item > items_;
+    size_t              bytes_ = 0;
+};
 
 }  // namespace
 
@@ -244,18 +268,28 @@ __global__ void triangle_kernel( int N, size_t triangles, const double* __restri
     }
 }
 
-int build_mass_tables( tn_mesh* m ); // mass.cu
+size_t mass_table_words( const tn_mesh* m, bool radial ); // mass.cu
+bool   fill_mass_tables( const tn_mesh* m );
 
-// both tables of cell.cuh, complete for every stream on return
-int build_triangle_tables( tn_mesh* m )
+// entries of a table of cell.cuh
+size_t triangle_words( const tn_mesh* m )
 {
-    const size_t   n = size_t( m->nd ) * m->N * m->N * 2, count = n * kTriangle + n / 2 + 4 * size_t( m->N );
+    const size_t n = size_t( m->nd ) * m->N * m->N * 2;
+    return n * kTriangle + n / 2 + 4 * size_t( m->N );
+}
+// fills the tables that are formed with the mesh; complete for every stream on return
+int fill_tables( tn_mesh* m )
+{
+    const size_t   n      = size_t( m->nd ) * m->N * m->N * 2;
     const unsigned blocks = unsigned( ( n + 127 ) / 128 );
-    TN_CUDA_TRY( cudaMalloc( &m->d_triangles, count * ( sizeof( double ) + sizeof( float ) ) ) );
-    m->d_triangles32 = reinterpret_cast< float* >( m->d_triangles + count );
     triangle_kernel< double ><<< blocks, 128 >>>( m->N, n, m->d_coords, m->d_radii, m->d_triangles );
     triangle_kernel< float ><<< blocks, 128 >>>( m->N, n, m->d_coords, m->d_radii, m->d_triangles32 );
     TN_LAUNCH_CHECK();
+    if ( !fill_mass_tables( m ) )
+    {
+        set_error( "tn_mesh_create: launching the mass stencils failed" );
+        return TN_ERR_CUDA;
+    }
     TN_CUDA_TRY( cudaStreamSynchronize( nullptr ) );
     return TN_OK;
 }
@@ -443,25 +477,33 @@ int mesh_create_diamonds( const ShellTopology& t, double r_min, double r_max, in
         std::memset( node_owned.data() + l * m->n1, m->h_lat_owned[l], m->n1 );
     int rc;
     std::vector< float > c32( m->h_coords.begin(), m->h_coords.end() ), r32( m->h_radii.begin(), m->h_radii.end() );
-    if ( ( rc = upload( m->h_coords.data(), m->h_coords.size(), &m->d_coords ) ) ||
-         ( rc = upload( m->h_radii.data(), m->h_radii.size(), &m->d_radii ) ) ||
-         ( rc = upload( c32.data(), c32.size(), &m->d_coords32 ) ) ||
-         ( rc = upload( r32.data(), r32.size(), &m->d_radii32 ) ) ||
-         ( rc = upload( m->h_lat_owned.data(), m->h_lat_owned.size(), &m->d_lat_owned ) ) ||
-         ( rc = upload( node_owned.data(), node_owned.size(), &m->d_node_owned ) ) ||
-         ( rc = upload( offsets.data(), offsets.size(), &m->d_halo_offsets ) ) ||
-         ( nd == kDiamonds && ( rc = upload( t.fv_ghost.data(), t.fv_ghost.size(), &m->d_fv_ghost ) ) ) ||
-         ( rc = upload( members.data(), members.size(), &m->d_halo_members ) ) ||
-         ( rc = upload( lat_group.data(), lat_group.size(), &m->d_lat_group ) ) || ( rc = build_triangle_tables( m ) ) ||
-         ( rc = build_mass_tables( m ) ) )
+    MeshArrays arrays;
+    arrays.place( m->d_coords, m->h_coords.size(), m->h_coords.data() );
+    arrays.place( m->d_radii, m->h_radii.size(), m->h_radii.data() );
+    arrays.place( m->d_coords32, c32.size(), c32.data() );
+    arrays.place( m->d_radii32, r32.size(), r32.data() );
+    arrays.place( m->d_lat_owned, m->h_lat_owned.size(), m->h_lat_owned.data() );
+    arrays.place( m->d_node_owned, node_owned.size(), node_owned.data() );
+    arrays.place( m->d_halo_offsets, offsets.size(), offsets.data() );
+    if ( nd == kDiamonds )
+        arrays.place( m->d_fv_ghost, t.fv_ghost.size(), t.fv_ghost.data() );
+    arrays.place( m->d_halo_members, members.size(), members.data() );
+    arrays.place( m->d_lat_group, lat_group.size(), lat_group.data() );
+    arrays.place( m->d_triangles, triangle_words( m ) );
+    arrays.place( m->d_triangles32, triangle_words( m ) );
+    arrays.place( m->mass_tables.lat, mass_table_words( m, false ) );
+    arrays.place( m->mass_tables.rad, mass_table_words( m, true ) );
+    arrays.place( m->mass_tables.lat32, mass_table_words( m, false ) );
+    arrays.place( m->mass_tables.rad32, mass_table_words( m, true ) );
+    arrays.place( m->d_red_partials, size_t( kRedMaxBlocks ) * 8 );
+    arrays.place( m->d_red_result, size_t( 16 ) );
+    arrays.place( m->d_red_counter, size_t( 1 ) );
+    if ( ( rc = arrays.allocate( &m->d_block ) ) || ( rc = fill_tables( m ) ) )
     {
         tn_mesh_destroy( m );
         return rc;
     }
-    if ( cudaMalloc( &m->d_red_partials, sizeof( double ) * kRedMaxBlocks * 8 ) != cudaSuccess ||
-         cudaMalloc( &m->d_red_result, sizeof( double ) * 16 ) != cudaSuccess ||
-         cudaMalloc( &m->d_red_counter, sizeof( unsigned int ) ) != cudaSuccess ||
-         cudaMallocHost( &m->h_red_result, sizeof( double ) * 16 ) != cudaSuccess ||
+    if ( cudaMallocHost( &m->h_red_result, sizeof( double ) * 16 ) != cudaSuccess ||
          cudaMemset( m->d_red_counter, 0, sizeof( unsigned int ) ) != cudaSuccess ||
          cudaStreamCreateWithFlags( &m->side_stream, cudaStreamNonBlocking ) != cudaSuccess ||
          cudaEventCreateWithFlags( &m->ev_fork, cudaEventDisableTiming ) != cudaSuccess ||
@@ -491,29 +533,12 @@ extern "C" int tn_mesh_destroy( tn_mesh* m )
 {
     if ( !m )
         return TN_OK;
-    cudaFree( m->d_coords );
-    cudaFree( m->d_radii );
-    cudaFree( m->d_coords32 );
-    cudaFree( m->d_radii32 );
-    cudaFree( m->d_lat_owned );
-    cudaFree( m->d_node_owned );
-    cudaFree( m->d_halo_offsets );
-    cudaFree( m->d_halo_members );
-    cudaFree( m->d_lat_group );
-    cudaFree( m->d_fv_ghost );
+    cudaFree( m->d_block );
     cudaFree( m->d_fv_orient );
-    for ( tn_lateral_tables* t : { &m->laplace_tables, &m->mass_tables } )
-    {
-        cudaFree( t->lat );
-        cudaFree( t->rad );
-        cudaFree( t->lat32 );
-        cudaFree( t->rad32 );
-    }
+    for ( void* p : { static_cast< void* >( m->laplace_tables.lat ), static_cast< void* >( m->laplace_tables.rad ),
+                      static_cast< void* >( m->laplace_tables.lat32 ), static_cast< void* >( m->laplace_tables.rad32 ) } )
+        cudaFree( p );
     cudaFree( m->d_work );
-    cudaFree( m->d_triangles );
-    cudaFree( m->d_red_partials );
-    cudaFree( m->d_red_result );
-    cudaFree( m->d_red_counter );
     if ( m->h_red_result )
         cudaFreeHost( m->h_red_result );
     if ( m->side_stream )
