@@ -21,7 +21,7 @@
 // by add_column.  Cells of a boundary layer with a condition are left to the first
 // blocks of the launch (one thread per lateral cell, wedge and side), which add the boundary
 // terms: with the lanes along r, every warp would otherwise carry that code for
-// one lane.  Level-6 free-slip FP64: 612 -> 132 us, FP32 276 -> 95 us.
+// one lane.  Level-6 free-slip FP64: 612 -> 127 us, FP32 276 -> 87 us.
 // Without communication the result is the derivative with respect to each
 // stored copy of k (each diamond's wedges use their own copy); with the
 // additive halo it is the derivative with respect to the unique node's value,

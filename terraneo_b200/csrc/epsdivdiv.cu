@@ -21,7 +21,7 @@
 // nodes are handed to the lane above, 12 atomics per cell.  Nodes that the
 // boundary treatment decouples enter with zero; their diagonal comes from
 // further blocks of the launch (one thread per lateral cell, wedge and side).
-// Level-6 apply with its halo: FP64 1,067 -> 256 us, FP32 577 -> 176 us, bound by
+// Level-6 apply with its halo: FP64 1,067 -> 246 us, FP32 577 -> 153 us, bound by
 // instruction issue; four resident blocks per SM (128 registers, some spilled)
 // beat three (168) by 5 % and two by 20 %.
 #include "cell.cuh"

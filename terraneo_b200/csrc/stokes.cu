@@ -34,8 +34,8 @@
 // One thread per fine cell, r fastest.  In B the two fine cells of one coarse
 // cell (neighbouring lanes) add together and hand their upper coarse nodes to
 // the next pair; in B^T the upper fine nodes go to the lane above (add_column).
-// Free-slip applies, FP64: B 288 -> 110 us and B^T 208 -> 132 us at level 6, 1,778 ->
-// 686 and 1,479 -> 972 us at level 7; bound by instruction issue (53 and 59 % of the
+// Free-slip applies, FP64: B 288 -> 109 us and B^T 208 -> 127 us at level 6, 1,778 ->
+// 719 and 1,479 -> 968 us at level 7; bound by instruction issue (53 and 59 % of the
 // slots), B^T also by its 12 atomics per cell.
 #include <cmath>
 

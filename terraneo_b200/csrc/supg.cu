@@ -28,7 +28,7 @@
 // entries alone.
 //
 // One thread per cell, lanes along r, contributions added by add_column, then
-// the additive halo sum.  Level-6 apply: FP64 1,522 -> 460 us, FP32 620 -> 242 us
+// the additive halo sum.  Level-6 apply: FP64 1,480 -> 457 us, FP32 620 -> 208 us
 // (half of what is left is tau: a root, an exponential and a division at each of
 // twelve points per cell).
 #include <cmath>
