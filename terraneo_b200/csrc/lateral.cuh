@@ -132,6 +132,16 @@ __device__ __forceinline__ void lateral_layer( int mode, const T ( &rad )[OP::R]
     }
 }
 
+// *p = v, or added to *p: as one atomic, so that applies on several streams may add into the same field
+template < typename T >
+__device__ __forceinline__ void lateral_store( T* p, T v, int add )
+{
+    if ( add )
+        atomicAdd( p, v );
+    else
+        *p = v;
+}
+
 template < typename OP, bool CG, typename T >
 __device__ __forceinline__ void lateral_tile( const LateralParams< T >& P, const LateralCG& cg, T beta, unsigned block, T* smem,
                                               Neumaier& dot )
@@ -284,7 +294,7 @@ __device__ __forceinline__ void lateral_tile( const LateralParams< T >& P, const
 #pragma unroll
                 for ( int cy = 0; cy < kTileY; ++cy, g += n1 )
                     if ( cy < ymax )
-                        *g = P.add ? *g + c[cy * kStride] : c[cy * kStride];
+                        lateral_store( g, c[cy * kStride], P.add );
             }
         }
     }
@@ -384,10 +394,9 @@ __device__ __forceinline__ void lateral_edge( const LateralParams< T >& P, const
     T* dst = P.dst.at( blockIdx.y );
     for ( int m = m0; m < m1; ++m )
     {
-        T* p = dst + size_t( P.members[m] ) * n1 + r;
         if ( CG && !cg.live )
             break;
-        *p = P.add ? *p + v : v;
+        lateral_store( dst + size_t( P.members[m] ) * n1 + r, v, P.add );
     }
 }
 

@@ -65,3 +65,28 @@ def test_first_mass_apply_in_a_capture():
     shell.apply(shell.KMass(pm), src, ref)
     torch.cuda.synchronize()
     assert torch.equal(dst.data, ref.data)
+
+
+@pytest.mark.parametrize("dtype,tol", [(torch.float64, 1e-13), (torch.float32, 1e-5)])
+def test_add_mode_from_two_streams(dtype, tol):
+    """applies on several streams that add into one field without communication lose no term: each of the 32 is a
+    thirty-second of the sum, far above the tolerance"""
+    from terraneo_b200 import shell, _capi as C
+    pm, n = shell.ShellMesh(5), 16
+    src, dst, once = (shell.VectorQ1Scalar(pm, dtype) for _ in range(3))
+    src.data.uniform_()
+    shell.apply(shell.KMass(pm, None, 0, C.APPLY_REPLACE, C.COMM_SKIP), src, once)
+    add = shell.KMass(pm, None, 0, C.APPLY_ADD, C.COMM_SKIP)
+    dst.data.zero_()
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    for s in streams:
+        with torch.cuda.stream(s):
+            torch.cuda._sleep(5_000_000)  # both queues fill before either runs
+    for _ in range(n):
+        for s in streams:
+            with torch.cuda.stream(s):
+                shell.apply(add, src, dst)
+    torch.cuda.synchronize()
+    want = 2 * n * once.data.double()
+    assert float((dst.data.double() - want).norm() / want.norm()) <= tol
