@@ -100,7 +100,6 @@ struct LateralParams
 // while it is read and written to p_new, and <p, A p> is summed over the owned nodes.
 struct LateralCG
 {
-    bool          live; // false: the stopping rule has fired, nothing is written
     const double* r;
     const double* p_old;
     double*       p_new;
@@ -281,7 +280,7 @@ __device__ __forceinline__ void lateral_tile( const LateralParams< T >& P, const
                 double   part[2] = { 0.0, 0.0 }; // plain sums per thread (two chains), compensated across threads
 #pragma unroll
                 for ( int cy = 0; cy < kTileY; ++cy, g += n1, q += n1 )
-                    if ( cy < ymax && cg.live )
+                    if ( cy < ymax )
                     {
                         *g = c[cy * kStride];
                         *q = v[cy * kStride];
@@ -338,8 +337,7 @@ __device__ __forceinline__ void lateral_edge( const LateralParams< T >& P, const
         const T         v0[3] = { value( u + rd ), value( u ), value( u + ru ) };
         if constexpr ( CG )
         {
-            if ( cg.live )
-                cg.p_new[u] = v0[1];
+            cg.p_new[u] = v0[1];
             owner = m == m0 ? v0[1] : owner;
         }
 #pragma unroll
@@ -393,11 +391,7 @@ __device__ __forceinline__ void lateral_edge( const LateralParams< T >& P, const
         dot.add( owner * v );
     T* dst = P.dst.at( blockIdx.y );
     for ( int m = m0; m < m1; ++m )
-    {
-        if ( CG && !cg.live )
-            break;
         lateral_store( dst + size_t( P.members[m] ) * n1 + r, v, P.add );
-    }
 }
 
 // shared memory of a tile block: operands, results and radial factors

@@ -7,9 +7,13 @@
 //   tn_pcg_update: x, r, |r|, the stopping rule and beta (krylov.cu).
 // The steps are those of tn_pcg_* (pcg.hpp:78-102 with z = r): every kernel returns
 // at once when the stopping rule has fired, so the host runs ahead of the device
-// and looks at the flag of the round before.  Per iteration: the Laplacian at level 5
-// 38 us of kernels (apply, halo, product, update, direction; 61 us with the gaps) ->
-// 24 us, the mass matrix at level 6 350 us with two host reads -> 80 us.
+// and looks at the flag some steps later.  A step issued after the rule has fired costs
+// its two launches, 9 us at level 6 (45 us when it read its operands and left out the
+// writes only); a step of a solve takes 0.5 % longer for waiting on the flag first at
+// level 6, no longer at level 5.
+// Per iteration: the Laplacian at level 5 38 us of kernels (apply, halo, product,
+// update, direction; 61 us with the gaps) -> 24 us, the mass matrix at level 6 350 us
+// with two host reads -> 80 us.
 #pragma once
 
 #include "lateral.cuh"
@@ -20,16 +24,15 @@ template < typename OP >
 __global__ void __launch_bounds__( kLateralThreads, 4 ) lateral_cg_kernel( LateralParams< double > P, LateralCG cg )
 {
     extern __shared__ double lateral_smem[];
-    // The flag is not waited for: the operands are loaded meanwhile, and only the writes depend on it.
-    cg.live           = cg.state[4] == 0.0; // not done
+    if ( cg.state[4] != 0.0 ) // done
+        return;
     const double beta = cg.state[3];
     Neumaier     dot;
     if ( blockIdx.x < P.edge_blocks )
         lateral_edge< OP, true >( P, cg, beta, blockIdx.x, dot );
     else
         lateral_tile< OP, true >( P, cg, beta, blockIdx.x - P.edge_blocks, lateral_smem, dot );
-    if ( cg.live )
-        block_sum_finish< 1 >( &dot, cg.partials, cg.counter, cg.state + 1 ); // pap
+    block_sum_finish< 1 >( &dot, cg.partials, cg.counter, cg.state + 1 ); // pap
 }
 
 // doubles of the work array of lateral_cg besides its four fields r, p, p', ap
@@ -78,8 +81,8 @@ int lateral_cg( const tn_mesh* m, LateralParams< double > P, const double* b, do
     if ( ( rc = tn_vec_lincomb_f64( m, 1, rr, 0.0, 2, c, bx, st ) ) ||
          ( rc = tn_pcg_begin_f64( 1, mm, rr, pp, cg.state, atol, st ) ) )
         return rc;
-    // the stopping flag travels to a pinned slot, every eighth step, and is looked at one round later (the slot, like the
-    // partial sums of tn_pcg_*, is the mesh's: one reduction or solve on a mesh at a time)
+    // the stopping flag travels to a pinned slot before steps 2, 8, 16, ... and is looked at before the next of these (the
+    // slot, like the partial sums of tn_pcg_*, is the mesh's: one reduction or solve on a mesh at a time)
     constexpr int kEvery = 8;
     cudaEvent_t   ev     = nullptr;
     TN_CUDA_TRY( cudaEventCreateWithFlags( &ev, cudaEventDisableTiming ) );
@@ -87,7 +90,7 @@ int lateral_cg( const tn_mesh* m, LateralParams< double > P, const double* b, do
     bool          pending = false;
     for ( int it = 0; it < max_iterations && rc == TN_OK; ++it )
     {
-        if ( it % kEvery == 0 )
+        if ( it == 2 || ( it > 0 && it % kEvery == 0 ) )
         {
             if ( pending && cudaEventSynchronize( ev ) == cudaSuccess && *static_cast< volatile double* >( flag ) != 0.0 )
                 break;

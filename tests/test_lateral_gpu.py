@@ -90,3 +90,35 @@ def test_add_mode_from_two_streams(dtype, tol):
     torch.cuda.synchronize()
     want = 2 * n * once.data.double()
     assert float((dst.data.double() - want).norm() / want.norm()) <= tol
+
+
+@pytest.mark.parametrize("solve", ["laplace", "projection"])
+def test_cg_steps_after_convergence_are_nearly_free(solve):
+    """a relative tolerance of 1e30 is met by the first step: the steps the host issued meanwhile cost little beside real
+    ones (a quarter is the bound; half when they read their operands all the same)"""
+    import time
+    from terraneo_b200 import shell
+    pm = shell.ShellMesh(6)
+    b, x = shell.VectorQ1Scalar(pm), shell.VectorQ1Scalar(pm)
+    b.data.normal_()
+    b.data[..., 0] = b.data[..., -1] = 0.0
+    fv = torch.randn((10,) + (pm.n1 + 1,) * 3, dtype=torch.float64, device="cuda")
+    work = torch.empty(5 * pm.stored_nodes, dtype=torch.float64, device="cuda")
+
+    def seconds(its, rtol):
+        best = 1e9
+        for _ in range(8):
+            x.data.zero_()
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            if solve == "laplace":
+                n, _ = shell.laplace_pcg(pm, b, x, its, rtol)
+            else:
+                n = shell.l2_project_fv_to_fe(pm, fv, x, False, its, rtol, 1e-300, work)
+            torch.cuda.synchronize()
+            best = min(best, time.perf_counter() - t)
+        assert n == (1 if rtol > 1 else its)
+        return best
+
+    one = seconds(1, 1e30)
+    assert seconds(16, 1e30) - one <= 0.25 * (seconds(16, 1e-300) - one)
