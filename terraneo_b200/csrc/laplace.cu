@@ -261,6 +261,7 @@ struct LaplaceOp
 {
     static constexpr int           S = 2, D = 2, K = S + D, R = 5;
     static constexpr bool          kDiff = true;
+    static constexpr bool          kExactDot = false; // <p, A p> summed as tn_pcg_pap sums it
     static __device__ __forceinline__ void layer( const T ( &f )[R], const T ( &b )[S], const T ( &t )[S], const T ( &d )[D + 1],
                                                   T& low, T& high )
     {

@@ -277,14 +277,17 @@ __device__ __forceinline__ void lateral_tile( const LateralParams< T >& P, const
             {
                 T*       q = cg.p_new + ( g - P.dst.p[0] );
                 const T* v = in + ( ( cx + 1 ) * ( kTileY + 2 ) + 1 ) * kStride + hl + 1;
-                double   part[2] = { 0.0, 0.0 }; // plain sums per thread (two chains), compensated across threads
+                double   part[2] = { 0.0, 0.0 }; // plain sums per thread: two chains, compensated across threads
 #pragma unroll
                 for ( int cy = 0; cy < kTileY; ++cy, g += n1, q += n1 )
                     if ( cy < ymax )
                     {
                         *g = c[cy * kStride];
                         *q = v[cy * kStride];
-                        part[cy & 1] += c[cy * kStride] * v[cy * kStride];
+                        if constexpr ( OP::kExactDot )
+                            dot.add( __dmul_rn( c[cy * kStride], v[cy * kStride] ) );
+                        else
+                            part[cy & 1] += c[cy * kStride] * v[cy * kStride];
                     }
                 dot.add( part[0] + part[1] );
             }

@@ -3,7 +3,8 @@
 //   lateral_cg_kernel: p = r + beta p, ap = A p and <p, ap> in one pass: the tile
 //     blocks form the new direction while they stage its operands (so it is never
 //     read back), write it to the other of two direction fields and sum the
-//     product while they write ap out; the halo is part of the apply;
+//     product while they write ap out (every term compensated where OP::kExactDot,
+//     else plainly per thread); the halo is part of the apply;
 //   tn_pcg_update: x, r, |r|, the stopping rule and beta (krylov.cu).
 // The steps are those of tn_pcg_* (pcg.hpp:78-102 with z = r): every kernel returns
 // at once when the stopping rule has fired, so the host runs ahead of the device

@@ -97,6 +97,7 @@ struct MassOp
 {
     static constexpr int           S = 1, D = 0, K = 1, R = 3;
     static constexpr bool          kDiff = false;
+    static constexpr bool          kExactDot = true; // <p, A p> of the projection's CG: 20 steps at level 6 take 1 % longer
     static __device__ __forceinline__ void layer( const T ( &f )[R], const T ( &b )[S], const T ( &t )[S], const T ( & )[D + 1],
                                                   T& low, T& high )
     {

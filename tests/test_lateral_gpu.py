@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from helpers import rel
-from oracle_lib import Mesh
+from oracle_lib import Mesh, pcg
 
 pytestmark = pytest.mark.gpu
 
@@ -122,3 +122,41 @@ def test_cg_steps_after_convergence_are_nearly_free(solve):
 
     one = seconds(1, 1e30)
     assert seconds(16, 1e30) - one <= 0.25 * (seconds(16, 1e-300) - one)
+
+
+def _row_pattern(om):
+    """A direction whose <p, A p> a plain sum along y gets wrong: in every row of interior columns one node of size one,
+    then seven whose terms are each just below half a unit in the last place of the first one's"""
+    import math
+    ones, e = np.ones(om.shape), np.zeros(om.shape)
+    s = np.full(om.shape, 2.0 ** -27)
+    for _ in range(3):
+        e[:, 1:-1, 1, 1:-1] = 1.0
+        e[:, 1:-1, 3::2, 1:-1] = s[:, 1:-1, 3::2, 1:-1]
+        e[:, :, -1] = 0.0
+        terms = e * om.kmass(ones, e, 0)
+        want = 0.95 * 2.0 ** -54 * terms[:, 1:-1, 1:2, 1:-1]
+        s[:, 1:-1, 3:-1:2, 1:-1] *= np.sqrt(want / terms[:, 1:-1, 3:-1:2, 1:-1])
+    return e, ones, lambda p, q: math.fsum((p * q)[om.omask == 1])
+
+
+def test_projection_sums_every_product():
+    """alpha = <r, r> / <p, A p> of the projection's first CG step, read off thousands of nodes, against exact sums of the
+    rounded products: one unit in the last place; seven terms lost per row would move it by 3.5e-16"""
+    from terraneo_b200 import shell
+    om, pm = Mesh(4), shell.ShellMesh(4)
+    e, ones, dot = _row_pattern(om)
+    x0, _ = pcg(lambda v: om.kmass(ones, v, 0), om.dot, -e, 200, 1e-17)  # the residual of an empty right-hand side is e
+    mass = shell.KMass(pm)
+    x, p, ap = (shell.VectorQ1Scalar(pm) for _ in range(3))
+    x.set_numpy(x0)
+    shell.apply(mass, x, p)
+    p.data.neg_()
+    shell.apply(mass, p, ap)
+    pn, apn = p.numpy()[0], ap.numpy()[0]
+    assert rel(pn, e) <= 1e-12
+    shell.l2_project_fv_to_fe(pm, torch.zeros((10,) + (om.N + 2,) * 3, dtype=torch.float64, device="cuda"), x,
+                              max_iterations=1, relative_tolerance=0.0, absolute_tolerance=0.0)
+    step = (x.numpy()[0].astype(np.longdouble) - x0)[pn > 0.5] / pn[pn > 0.5]
+    alpha = dot(pn, pn) / dot(pn, apn)
+    assert abs(float(step.mean() / alpha - 1)) <= 2.0 ** -52
