@@ -285,6 +285,8 @@ struct LaplaceOp
     {
         return f[0] * v[0] + f[2] * v[2] + f[4] * ( v[3] + v[1] );
     }
+    using Sum = double;
+    static __device__ double entry( double a, int ) { return a; }
     // adds the factors between vertices i and j of a triangle
     static __device__ void triangle( const double* p0, const double* p1, const double* p2, int i, int j, double* A )
     {

@@ -471,8 +471,40 @@ int launch_lateral( const tn_mesh* m, LateralParams< T > P, int nc, int apply_mo
     return TN_OK;
 }
 
-// Tabulates an operator's stencils ([7 K][column], thread per column: OP::triangle gives the factors between two
-// vertices of a triangle) and radial factors ([R][layer], OP::radial).
+// Unevaluated sum of two doubles (v the rounded sum), for tables whose entries are to carry no more than their own
+// rounding: error-free sums (Knuth's two-sum) and products (fused multiply-add).
+struct Pair
+{
+    double v = 0.0, e = 0.0;
+};
+__device__ __forceinline__ Pair pair_sum( double a, double b )
+{
+    const double s = a + b, z = s - a;
+    return { s, ( a - ( s - z ) ) + ( b - z ) };
+}
+__device__ __forceinline__ Pair operator+( const Pair& a, const Pair& b )
+{
+    const Pair s = pair_sum( a.v, b.v );
+    return pair_sum( s.v, s.e + ( a.e + b.e ) );
+}
+__device__ __forceinline__ Pair operator-( const Pair& a )
+{
+    return { -a.v, -a.e };
+}
+__device__ __forceinline__ Pair operator*( const Pair& a, const Pair& b )
+{
+    const double p = __dmul_rn( a.v, b.v );
+    return pair_sum( p, fma( a.v, b.v, -p ) + ( a.v * b.e + a.e * b.v ) );
+}
+// a / d rounded once (but for ties)
+__device__ __forceinline__ double quotient( const Pair& a, double d )
+{
+    const double q = a.v / d;
+    return q + ( fma( -q, d, a.v ) + a.e ) / d;
+}
+
+// Tabulates an operator's stencils ([7 K][column], thread per column: OP::triangle adds the factors between two
+// vertices of a triangle, OP::entry is the value of their sum) and radial factors ([R][layer], OP::radial).
 template < typename OP, typename T >
 __global__ void lateral_table_kernel( int N, size_t columns, const double* __restrict__ coords,
                                       const double* __restrict__ radii, T* lat, T* rad )
@@ -489,10 +521,7 @@ __global__ void lateral_table_kernel( int N, size_t columns, const double* __res
     if ( col >= columns )
         return;
     const int y = int( col % n1 ), x = int( col / n1 % n1 );
-    double    A[kStencil][OP::K];
-    for ( int e = 0; e < kStencil; ++e )
-        for ( int k = 0; k < OP::K; ++k )
-            A[e][k] = 0.0;
+    typename OP::Sum A[kStencil][OP::K] = {};
     for ( int w = 0; w < 2; ++w )
         for ( int i = 0; i < 3; ++i )
         {
@@ -515,7 +544,7 @@ __global__ void lateral_table_kernel( int N, size_t columns, const double* __res
         }
     for ( int e = 0; e < kStencil; ++e )
         for ( int k = 0; k < OP::K; ++k )
-            lat[size_t( e * OP::K + k ) * columns + col] = T( A[e][k] );
+            lat[size_t( e * OP::K + k ) * columns + col] = T( OP::entry( A[e][k], e ) );
 }
 
 // the double or single precision member of a table pair

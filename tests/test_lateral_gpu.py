@@ -160,3 +160,51 @@ def test_projection_sums_every_product():
     step = (x.numpy()[0].astype(np.longdouble) - x0)[pn > 0.5] / pn[pn > 0.5]
     alpha = dot(pn, pn) / dot(pn, apn)
     assert abs(float(step.mean() / alpha - 1)) <= 2.0 ** -52
+
+
+def _mass_factors(om):
+    """lateral stencil {offset: [10, N-1, N-1]} of the interior columns and radial factors [3][N] of the mass matrix in
+    extended precision (the 3x2 rule: lateral points (2/3, 1/6), (1/6, 2/3), (1/6, 1/6), zeta = -+1/sqrt(3), weights 1/6)"""
+    N, LD, lat = om.N, np.longdouble, {}
+    P, r = om.coords.astype(LD), om.radii[0].astype(LD)
+    for nodes in (((0, 0), (1, 0), (0, 1)), ((1, 1), (0, 1), (1, 0))):
+        p = [P[:, x:x + N, y:y + N] for x, y in nodes]
+        D = np.abs((np.cross(p[1] - p[0], p[2] - p[0]) * p[0]).sum(-1))
+        for i, a in enumerate(nodes):
+            for j, b in enumerate(nodes):
+                e = lat.setdefault((b[0] - a[0], b[1] - a[1]), np.zeros(P.shape[:3], LD))
+                e[:, a[0]:a[0] + N, a[1]:a[1] + N] += D / (12 if i == j else 24)
+    h, g, f = (r[1:] - r[:-1]) / 2, 1 / np.sqrt(LD(3)), np.zeros((3, N), LD)
+    for z in (-g, g):
+        n, rr = ((1 - z) / 2, (1 + z) / 2), r[:-1] + h * (1 + z)
+        for k in range(3):
+            f[k] += h * rr * rr * n[k // 2] * n[(k + 1) // 2]
+    return {e: v[:, 1:-1, 1:-1] for e, v in lat.items()}, f
+
+
+@pytest.mark.parametrize("L,rmin", [(3, 0.55), (4, 0.35), (4, 0.55)])
+def test_mass_tables_are_rounded_once(L, rmin):
+    """entries of the mass matrix, read off by fields that are one at every third node: stencil and radial factor carry
+    half a unit each, their product another (3 x 2^-53), and the node's own entry one for the sum of its two layers"""
+    from terraneo_b200 import shell
+    om, pm = Mesh(L, rmin), shell.ShellMesh(L, rmin, 1.0)
+    lat, f = _mass_factors(om)
+    N, op = om.N, shell.KMass(pm)
+    src, dst = shell.VectorQ1Scalar(pm), shell.VectorQ1Scalar(pm)
+    own = np.zeros(N + 1, np.longdouble)
+    own[:-1] += f[0]
+    own[1:] += f[2]
+    worst = [0.0, 0.0]
+    for a, b, c in np.ndindex(3, 3, 3):
+        u = np.zeros(om.shape)
+        u[:, a::3, b::3, c::3] = 1.0
+        src.set_numpy(u)
+        shell.apply(op, src, dst)
+        got = dst.numpy()[0][:, 1:-1, 1:-1]
+        for (dx, dy), s in lat.items():
+            at = u[:, 1 + dx:N + dx, 1 + dy:N + dy] != 0.0  # columns whose neighbour (dx, dy) holds ones, at their levels
+            for k, (here, want) in enumerate(((at, s[..., None] * own),
+                                              (at[..., :-1], s[..., None] * f[1]), (at[..., 1:], s[..., None] * f[1]))):
+                out = got if k == 0 else (got[..., 1:] if k == 1 else got[..., :-1])
+                worst[k > 0] = max(worst[k > 0], float(np.abs(out[here] / want[here] - 1).max(initial=0)))
+    assert worst[1] <= 3.01 * 2.0 ** -53 and worst[0] <= 4.01 * 2.0 ** -53, worst
