@@ -287,20 +287,25 @@ struct LaplaceOp
     }
     using Sum = double;
     static __device__ double entry( double a, int ) { return a; }
-    // adds the factors between vertices i and j of a triangle
-    static __device__ void triangle( const double* p0, const double* p1, const double* p2, int i, int j, double* A )
+    static __device__ void triangle( const double* p0, const double* p1, const double* p2, int i, const int ( &e )[3],
+                                     double ( &A )[kStencil][K] )
     {
         const LateralTriangle tri( p0, p1, p2 );
-        const double   vv = LateralTriangle::dot( tri.v, tri.v );
+        const double          vv = LateralTriangle::dot( tri.v, tri.v ), f = kFelippaW * tri.sig;
+#pragma unroll
         for ( int q = 0; q < 3; ++q )
         {
             double u[3][3], l[3];
             tri.at( felippa_xi( q ), felippa_eta( q ), u, l );
-            const double f = kFelippaW * tri.sig;
-            A[0] += f * LateralTriangle::dot( u[i], u[j] );
-            A[1] += f * LateralTriangle::dot( u[j], tri.v ) * l[i];
-            A[2] += f * l[i] * l[j] * vv;
-            A[3] += f * LateralTriangle::dot( u[i], tri.v ) * l[j];
+#pragma unroll
+            for ( int j = 0; j < 3; ++j )
+            {
+                double* a = A[e[j]];
+                a[0] += f * LateralTriangle::dot( u[i], u[j] );
+                a[1] += f * LateralTriangle::dot( u[j], tri.v ) * l[i];
+                a[2] += f * l[i] * l[j] * vv;
+                a[3] += f * LateralTriangle::dot( u[i], tri.v ) * l[j];
+            }
         }
     }
     static __device__ void radial( double r1, double r2, double* f )

@@ -62,6 +62,14 @@ constexpr int kStride   = ( kMaxRun + 2 ) | 1; // words per staged column
 __host__ __device__ constexpr int stencil_dx( int i ) { return i == 1 || i == 5 ? 1 : ( i == 2 || i == 6 ? -1 : 0 ); }
 __host__ __device__ constexpr int stencil_dy( int i ) { return i == 3 || i == 6 ? 1 : ( i == 4 || i == 5 ? -1 : 0 ); }
 
+__host__ __device__ constexpr int stencil_entry( int dx, int dy )
+{
+    for ( int i = 0; i < kStencil; ++i )
+        if ( stencil_dx( i ) == dx && stencil_dy( i ) == dy )
+            return i;
+    return -1;
+}
+
 // Coupling of a cell's wedge nodes: all (kNeu), CMB-side nodes decoupled
 // keeping their diagonal (kBot), SURFACE-side ones likewise (kTop), or the
 // diagonal alone (kDiag).  It depends on the cell's radial layer only.
@@ -145,7 +153,8 @@ template < typename OP, bool CG, typename T >
 __device__ __forceinline__ void lateral_tile( const LateralParams< T >& P, const LateralCG& cg, T beta, unsigned block, T* smem,
                                               Neumaier& dot )
 {
-    constexpr int K = OP::K, R = OP::R;
+    constexpr int  K = OP::K, R = OP::R;
+    constexpr bool exact_dot = CG && OP::kExactDot;
     const int     n1 = P.n1, tid = int( threadIdx.x ), lane = tid & 31, warp = tid >> 5;
     const int     chunk = int( block % unsigned( P.runs ) );
     const unsigned tile = block / unsigned( P.runs );
@@ -284,7 +293,7 @@ __device__ __forceinline__ void lateral_tile( const LateralParams< T >& P, const
                     {
                         *g = c[cy * kStride];
                         *q = v[cy * kStride];
-                        if constexpr ( OP::kExactDot )
+                        if constexpr ( exact_dot )
                             dot.add( __dmul_rn( c[cy * kStride], v[cy * kStride] ) );
                         else
                             part[cy & 1] += c[cy * kStride] * v[cy * kStride];
@@ -503,26 +512,41 @@ __device__ __forceinline__ double quotient( const Pair& a, double d )
     return q + ( fma( -q, d, a.v ) + a.e ) / d;
 }
 
-// Tabulates an operator's stencils ([7 K][column], thread per column: OP::triangle adds the factors between two
-// vertices of a triangle, OP::entry is the value of their sum) and radial factors ([R][layer], OP::radial).
-template < typename OP, typename T >
-__global__ void lateral_table_kernel( int N, size_t columns, const double* __restrict__ coords,
-                                      const double* __restrict__ radii, T* lat, T* rad )
+// Tabulates an operator's stencils ([7 K][column], thread per column: OP::triangle adds the factors between vertex i of
+// a triangle and its three to their entries, OP::entry is the value of such a sum) and radial factors ([R][layer],
+// OP::radial), in the precisions that are given an array.
+struct LateralTables
 {
+    double *lat, *rad;
+    float * lat32, *rad32;
+};
+template < typename OP >
+__global__ void __launch_bounds__( 128 ) lateral_table_kernel( int N, size_t columns, const double* __restrict__ coords,
+                                                              const double* __restrict__ radii, LateralTables t )
+{
+    const auto put = []( double* d, float* f, size_t i, double v ) {
+        if ( d )
+            d[i] = v;
+        if ( f )
+            f[i] = float( v );
+    };
     const size_t col = blockIdx.x * size_t( blockDim.x ) + threadIdx.x;
     const int    n1  = N + 1;
     if ( col < size_t( N ) )
     {
         double f[OP::R];
         OP::radial( radii[col], radii[col + 1], f );
+#pragma unroll
         for ( int i = 0; i < OP::R; ++i )
-            rad[size_t( i ) * N + col] = T( f[i] );
+            put( t.rad, t.rad32, size_t( i ) * N + col, f[i] );
     }
     if ( col >= columns )
         return;
     const int y = int( col % n1 ), x = int( col / n1 % n1 );
     typename OP::Sum A[kStencil][OP::K] = {};
+#pragma unroll
     for ( int w = 0; w < 2; ++w )
+#pragma unroll
         for ( int i = 0; i < 3; ++i )
         {
             // the triangle w whose vertex i is this column
@@ -530,21 +554,21 @@ __global__ void lateral_table_kernel( int N, size_t columns, const double* __res
             if ( cx < 0 || cy < 0 || cx >= N || cy >= N )
                 continue;
             const double* p[3];
-            for ( int j = 0; j < 3; ++j )
-                p[j] = coords + ( col + ptrdiff_t( wedge_node( w, j, 0 ) - wedge_node( w, i, 0 ) ) * n1 +
-                                  wedge_node( w, j, 1 ) - wedge_node( w, i, 1 ) ) * 3;
+            int           e[3];
+#pragma unroll
             for ( int j = 0; j < 3; ++j )
             {
                 const int dx = wedge_node( w, j, 0 ) - wedge_node( w, i, 0 ), dy = wedge_node( w, j, 1 ) - wedge_node( w, i, 1 );
-                int       e  = 0;
-                while ( stencil_dx( e ) != dx || stencil_dy( e ) != dy )
-                    ++e;
-                OP::triangle( p[0], p[1], p[2], i, j, A[e] );
+                p[j] = coords + ( col + ptrdiff_t( dx ) * n1 + dy ) * 3;
+                e[j] = stencil_entry( dx, dy );
             }
+            OP::triangle( p[0], p[1], p[2], i, e, A );
         }
+#pragma unroll
     for ( int e = 0; e < kStencil; ++e )
+#pragma unroll
         for ( int k = 0; k < OP::K; ++k )
-            lat[size_t( e * OP::K + k ) * columns + col] = T( OP::entry( A[e][k], e ) );
+            put( t.lat, t.lat32, size_t( e * OP::K + k ) * columns + col, OP::entry( A[e][k], e ) );
 }
 
 // the double or single precision member of a table pair
@@ -563,11 +587,11 @@ size_t lateral_table_words( const tn_mesh* m, bool radial )
 {
     return radial ? size_t( OP::R ) * m->N : size_t( kStencil * OP::K ) * m->nlat;
 }
-template < typename OP, typename T >
-bool lateral_fill( const tn_mesh* m, T* lat, T* rad, cudaStream_t st )
+template < typename OP >
+bool lateral_fill( const tn_mesh* m, const LateralTables& t, cudaStream_t st )
 {
     const size_t n = std::max( m->nlat, size_t( m->N ) );
-    lateral_table_kernel< OP, T ><<< unsigned( ( n + 127 ) / 128 ), 128, 0, st >>>( m->N, m->nlat, m->d_coords, m->d_radii, lat, rad );
+    lateral_table_kernel< OP ><<< unsigned( ( n + 127 ) / 128 ), 128, 0, st >>>( m->N, m->nlat, m->d_coords, m->d_radii, t );
     return cudaGetLastError() == cudaSuccess;
 }
 
@@ -590,7 +614,9 @@ bool lateral_tables( const tn_mesh* m, tn_lateral_tables tn_mesh::*which, Latera
             cudaFree( l );
             return false;
         }
-        if ( !lateral_fill< OP, T >( m, l, r, st ) || cudaStreamSynchronize( st ) != cudaSuccess )
+        LateralTables out{};
+        lateral_slot< T >( out.lat, out.lat32 ) = l, lateral_slot< T >( out.rad, out.rad32 ) = r;
+        if ( !lateral_fill< OP >( m, out, st ) || cudaStreamSynchronize( st ) != cudaSuccess )
         {
             (void) cudaGetLastError();
             cudaFree( l );

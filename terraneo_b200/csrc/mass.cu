@@ -114,17 +114,24 @@ struct MassOp
     // |D| of a triangle; the rule's sums of lat_i lat_j / 6 are 1/12 for i = j and else 1/24
     using Sum = Pair;
     static __device__ double entry( const Pair& a, int e ) { return quotient( a, e == 0 ? 12.0 : 24.0 ); }
-    static __device__ void   triangle( const double* p0, const double* p1, const double* p2, int, int, Pair* A )
+    static __device__ void   triangle( const double* p0, const double* p1, const double* p2, int, const int ( &e )[3],
+                                       Pair ( &A )[kStencil][K] )
     {
         Pair a[3], b[3], D;
+#pragma unroll
         for ( int k = 0; k < 3; ++k )
             a[k] = pair_sum( p1[k], -p0[k] ), b[k] = pair_sum( p2[k], -p0[k] );
+#pragma unroll
         for ( int k = 0; k < 3; ++k )
         {
             const int i = ( k + 1 ) % 3, j = ( k + 2 ) % 3;
             D           = D + ( a[i] * b[j] + -( a[j] * b[i] ) ) * Pair{ p0[k] };
         }
-        A[0] = A[0] + ( D.v < 0.0 ? -D : D );
+        if ( D.v < 0.0 )
+            D = -D;
+#pragma unroll
+        for ( int j = 0; j < 3; ++j )
+            A[e[j]][0] = A[e[j]][0] + D;
     }
     // h sum over zeta = -+1/sqrt(3) of r^2 n_li n_lj in closed form, m = r1 + h:
     // h (6 r1 m + 2 h^2) / 9, h (3 m^2 + h^2) / 9, h (6 r2 m + 2 h^2) / 9
@@ -179,8 +186,7 @@ size_t mass_table_words( const tn_mesh* m, bool radial ) { return lateral_table_
 bool   fill_mass_tables( const tn_mesh* m )
 {
     const tn_lateral_tables& t = m->mass_tables;
-    return lateral_fill< MassOp< double >, double >( m, t.lat, t.rad, nullptr ) &&
-           lateral_fill< MassOp< float >, float >( m, t.lat32, t.rad32, nullptr );
+    return lateral_fill< MassOp< double > >( m, LateralTables{ t.lat, t.rad, t.lat32, t.rad32 }, nullptr );
 }
 
 // CG on the plain mass matrix from x's values (lateral_cg.cuh); fields: 4 stored-node fields

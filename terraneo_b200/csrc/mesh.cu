@@ -221,50 +221,59 @@ __device__ __forceinline__ double diff_of_products( double a, double b, double c
     return fma( a, b, -cd ) + err;
 }
 
-// Thread per triangle: beta_1, beta_2, v, 1 / D and the radial and volume factors (cell.cuh).  Every layer of a column
-// uses the same entry, so its rounding does not average out: the cross products are formed to the last bits, and
-// D = v . p0 with the products' errors.
-template < typename T >
-__global__ void triangle_kernel( int N, size_t triangles, const double* __restrict__ coords,
-                                 const double* __restrict__ radii, T* table )
+// Thread per lateral cell: beta_1, beta_2, v, 1 / D of its two triangles and the radial and volume factors (cell.cuh), in
+// both precisions.  Every layer of a column uses the same entry, so its rounding does not average out: the cross products
+// are formed to the last bits, and D = v . p0 with the products' errors.
+__global__ void __launch_bounds__( 128 ) triangle_kernel( int N, size_t cells, const double* __restrict__ coords,
+                                                         const double* __restrict__ radii, double* table, float* table32 )
 {
-    const size_t t = blockIdx.x * size_t( blockDim.x ) + threadIdx.x;
-    if ( t >= triangles )
+    const auto put = [=]( size_t i, double v ) { table[i] = v, table32[i] = float( v ); };
+    const size_t c = blockIdx.x * size_t( blockDim.x ) + threadIdx.x;
+    if ( c >= cells )
         return;
-    const int     w = int( t & 1 ), y = int( t / 2 % N ), x = int( t / 2 / N % N ), d = int( t / 2 / N / N ), n1 = N + 1;
-    const double* p[3];
-    for ( int i = 0; i < 3; ++i )
-        p[i] = coords + lat_index( n1, d, x + wedge_node( w, i, 0 ), y + wedge_node( w, i, 1 ) ) * 3;
-    double a[3], b[3], q[kTriangle], D = 0.0, err = 0.0;
-    for ( int k = 0; k < 3; ++k )
-        a[k] = p[1][k] - p[0][k], b[k] = p[2][k] - p[0][k];
-    for ( int k = 0; k < 3; ++k )
+    const int    y = int( c % N ), x = int( c / N % N ), d = int( c / N / N ), n1 = N + 1;
+    const size_t layers = cells * 2 * kTriangle, fv = layers + 3 * size_t( N );
+    double       volume = 0.0;
+#pragma unroll
+    for ( int w = 0; w < 2; ++w )
     {
-        const int i = ( k + 1 ) % 3, j = ( k + 2 ) % 3;
-        q[k]     = diff_of_products( b[i], p[0][j], b[j], p[0][i] );
-        q[3 + k] = diff_of_products( p[0][i], a[j], p[0][j], a[i] );
-        q[6 + k] = diff_of_products( a[i], b[j], a[j], b[i] );
-        const double pr = q[6 + k] * p[0][k], s = D + pr, z = s - D; // two-sum
-        err += fma( q[6 + k], p[0][k], -pr ) + ( ( D - ( s - z ) ) + ( pr - z ) );
-        D = s;
+        double p[3][3], a[3], b[3], q[kTriangle], D = 0.0, err = 0.0;
+#pragma unroll
+        for ( int i = 0; i < 3; ++i )
+#pragma unroll
+            for ( int k = 0; k < 3; ++k )
+                p[i][k] = coords[lat_index( n1, d, x + wedge_node( w, i, 0 ), y + wedge_node( w, i, 1 ) ) * 3 + k];
+#pragma unroll
+        for ( int k = 0; k < 3; ++k )
+            a[k] = p[1][k] - p[0][k], b[k] = p[2][k] - p[0][k];
+#pragma unroll
+        for ( int k = 0; k < 3; ++k )
+        {
+            const int i = ( k + 1 ) % 3, j = ( k + 2 ) % 3;
+            q[k]     = diff_of_products( b[i], p[0][j], b[j], p[0][i] );
+            q[3 + k] = diff_of_products( p[0][i], a[j], p[0][j], a[i] );
+            q[6 + k] = diff_of_products( a[i], b[j], a[j], b[i] );
+            const double pr = __dmul_rn( q[6 + k], p[0][k] ), s = D + pr, z = s - D; // two-sum
+            err += fma( q[6 + k], p[0][k], -pr ) + ( ( D - ( s - z ) ) + ( pr - z ) );
+            D = s;
+        }
+        q[9] = 1.0 / ( D + err );
+        volume += fabs( D + err );
+#pragma unroll
+        for ( int k = 0; k < kTriangle; ++k )
+            put( ( c * 2 + w ) * kTriangle + k, q[k] );
     }
-    q[9] = 1.0 / ( D + err );
-    for ( int k = 0; k < kTriangle; ++k )
-        table[t * kTriangle + k] = T( q[k] );
-    // FV cells: the lateral factor of the inverse volume is 1 / (|D_0| + |D_1|), with the partner's D from its thread
-    const double other = __shfl_xor_sync( __activemask(), fabs( D + err ), 1 );
-    T*           fv    = table + triangles * kTriangle + 3 * N;
-    if ( w == 0 )
-        fv[t / 2] = T( 1.0 / ( fabs( D + err ) + other ) );
-    if ( t < size_t( N ) )
+    // FV cells: the lateral factor of the inverse volume is 1 / (|D_0| + |D_1|)
+    put( fv + c, 1.0 / volume );
+    if ( c < size_t( N ) )
     {
         // h, r1 / h, r1 and the radial factor h / 2 (r(-g)^2 + r(g)^2) of the volume, g = 1 / sqrt(3)
-        const double r1 = radii[t], h = 0.5 * ( radii[t + 1] - r1 ), g = 0.5773502691896258;
+        const double r1 = radii[c], h = 0.5 * ( radii[c + 1] - r1 ), g = 0.5773502691896258;
         const double rm = r1 + h * ( 1.0 - g ), rp = r1 + h * ( 1.0 + g );
-        table[triangles * kTriangle + t]         = T( h );
-        table[triangles * kTriangle + N + t]     = T( r1 / h );
-        table[triangles * kTriangle + 2 * N + t] = T( r1 );
-        fv[triangles / 2 + t]                    = T( 1.0 / ( 0.5 * h * ( rm * rm + rp * rp ) ) );
+        put( layers + c, h );
+        put( layers + N + c, r1 / h );
+        put( layers + 2 * size_t( N ) + c, r1 );
+        put( fv + cells + c, 1.0 / ( 0.5 * h * ( rm * rm + rp * rp ) ) );
     }
 }
 
@@ -274,23 +283,21 @@ bool   fill_mass_tables( const tn_mesh* m );
 // entries of a table of cell.cuh
 size_t triangle_words( const tn_mesh* m )
 {
-    const size_t n = size_t( m->nd ) * m->N * m->N * 2;
-    return n * kTriangle + n / 2 + 4 * size_t( m->N );
+    const size_t cells = size_t( m->nd ) * m->N * m->N;
+    return cells * ( 2 * kTriangle + 1 ) + 4 * size_t( m->N );
 }
-// fills the tables that are formed with the mesh; complete for every stream on return
+// fills the tables that are formed with the mesh (both precisions in one launch each), on the default stream
 int fill_tables( tn_mesh* m )
 {
-    const size_t   n      = size_t( m->nd ) * m->N * m->N * 2;
-    const unsigned blocks = unsigned( ( n + 127 ) / 128 );
-    triangle_kernel< double ><<< blocks, 128 >>>( m->N, n, m->d_coords, m->d_radii, m->d_triangles );
-    triangle_kernel< float ><<< blocks, 128 >>>( m->N, n, m->d_coords, m->d_radii, m->d_triangles32 );
+    const size_t cells = size_t( m->nd ) * m->N * m->N;
+    triangle_kernel<<< unsigned( ( cells + 127 ) / 128 ), 128 >>>( m->N, cells, m->d_coords, m->d_radii, m->d_triangles,
+                                                                  m->d_triangles32 );
     TN_LAUNCH_CHECK();
     if ( !fill_mass_tables( m ) )
     {
         set_error( "tn_mesh_create: launching the mass stencils failed" );
         return TN_ERR_CUDA;
     }
-    TN_CUDA_TRY( cudaStreamSynchronize( nullptr ) );
     return TN_OK;
 }
 
@@ -507,9 +514,10 @@ int mesh_create_diamonds( const ShellTopology& t, double r_min, double r_max, in
          cudaMemset( m->d_red_counter, 0, sizeof( unsigned int ) ) != cudaSuccess ||
          cudaStreamCreateWithFlags( &m->side_stream, cudaStreamNonBlocking ) != cudaSuccess ||
          cudaEventCreateWithFlags( &m->ev_fork, cudaEventDisableTiming ) != cudaSuccess ||
-         cudaEventCreateWithFlags( &m->ev_join, cudaEventDisableTiming ) != cudaSuccess )
+         cudaEventCreateWithFlags( &m->ev_join, cudaEventDisableTiming ) != cudaSuccess ||
+         cudaStreamSynchronize( nullptr ) != cudaSuccess ) // the tables and the counter are complete for every stream
     {
-        set_error( "tn_mesh_create: device scratch, stream or event creation failed" );
+        set_error( "tn_mesh_create: device scratch, stream, event or table creation failed" );
         tn_mesh_destroy( m );
         return TN_ERR_NOMEM;
     }

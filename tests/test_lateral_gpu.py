@@ -208,3 +208,17 @@ def test_mass_tables_are_rounded_once(L, rmin):
                 out = got if k == 0 else (got[..., 1:] if k == 1 else got[..., :-1])
                 worst[k > 0] = max(worst[k > 0], float(np.abs(out[here] / want[here] - 1).max(initial=0)))
     assert worst[1] <= 3.01 * 2.0 ** -53 and worst[0] <= 4.01 * 2.0 ** -53, worst
+
+
+def test_mesh_tables_take_one_launch_each():
+    """what a mesh forms on the device, whatever it is used for: triangle vectors and mass stencils, both precisions at
+    once"""
+    from torch.profiler import ProfilerActivity, profile
+    from terraneo_b200 import shell
+    shell.ShellMesh(2)
+    with profile(activities=[ProfilerActivity.CUDA], acc_events=True) as prof:
+        mesh = shell.ShellMesh(3)
+        torch.cuda.synchronize()
+    del mesh
+    kernels = [e.name for e in prof.events() if "_kernel" in e.name]
+    assert len(kernels) == 2, kernels
