@@ -96,7 +96,7 @@ int mesh_create_diamonds( const ShellTopology& t, double r_min, double r_max, in
 }  // namespace tn
 
 // Lateral stencils and radial factors of an operator whose wedge matrices
-// separate (lateral.cuh), in double and single precision, built on first use.
+// separate (lateral.cuh), in double and single precision.
 struct tn_lateral_tables
 {
     double *lat = nullptr, *rad = nullptr;
@@ -139,8 +139,9 @@ struct tn_mesh
     // flipped (the orientation test against the neighbour's centre), built on first use
     uint8_t* d_fv_orient = nullptr;
 
-    tn_lateral_tables laplace_tables, mass_tables;
-    // wedge vectors per triangle (cell.cuh)
+    tn_lateral_tables laplace_tables; // built on first use
+    // formed with the mesh of a whole shell (a shard has neither): the mass matrix, wedge vectors per triangle (cell.cuh)
+    tn_lateral_tables mass_tables;
     double* d_triangles   = nullptr;
     float*  d_triangles32 = nullptr;
 

@@ -283,13 +283,13 @@ bool   fill_mass_tables( const tn_mesh* m );
 // entries of a table of cell.cuh
 size_t triangle_words( const tn_mesh* m )
 {
-    const size_t cells = size_t( m->nd ) * m->N * m->N;
+    const size_t cells = size_t( kDiamonds ) * m->N * m->N;
     return cells * ( 2 * kTriangle + 1 ) + 4 * size_t( m->N );
 }
-// fills the tables that are formed with the mesh (both precisions in one launch each), on the default stream
+// fills the tables that are formed with a whole shell's mesh (both precisions in one launch each), on the default stream
 int fill_tables( tn_mesh* m )
 {
-    const size_t cells = size_t( m->nd ) * m->N * m->N;
+    const size_t cells = size_t( kDiamonds ) * m->N * m->N;
     triangle_kernel<<< unsigned( ( cells + 127 ) / 128 ), 128 >>>( m->N, cells, m->d_coords, m->d_radii, m->d_triangles,
                                                                   m->d_triangles32 );
     TN_LAUNCH_CHECK();
@@ -492,20 +492,23 @@ int mesh_create_diamonds( const ShellTopology& t, double r_min, double r_max, in
     arrays.place( m->d_lat_owned, m->h_lat_owned.size(), m->h_lat_owned.data() );
     arrays.place( m->d_node_owned, node_owned.size(), node_owned.data() );
     arrays.place( m->d_halo_offsets, offsets.size(), offsets.data() );
-    if ( nd == kDiamonds )
-        arrays.place( m->d_fv_ghost, t.fv_ghost.size(), t.fv_ghost.data() );
     arrays.place( m->d_halo_members, members.size(), members.data() );
     arrays.place( m->d_lat_group, lat_group.size(), lat_group.data() );
-    arrays.place( m->d_triangles, triangle_words( m ) );
-    arrays.place( m->d_triangles32, triangle_words( m ) );
-    arrays.place( m->mass_tables.lat, mass_table_words( m, false ) );
-    arrays.place( m->mass_tables.rad, mass_table_words( m, true ) );
-    arrays.place( m->mass_tables.lat32, mass_table_words( m, false ) );
-    arrays.place( m->mass_tables.rad32, mass_table_words( m, true ) );
+    const bool whole = nd == kDiamonds; // what only the operators of the whole shell read is left out of a shard
+    if ( whole )
+    {
+        arrays.place( m->d_fv_ghost, t.fv_ghost.size(), t.fv_ghost.data() );
+        arrays.place( m->d_triangles, triangle_words( m ) );
+        arrays.place( m->d_triangles32, triangle_words( m ) );
+        arrays.place( m->mass_tables.lat, mass_table_words( m, false ) );
+        arrays.place( m->mass_tables.rad, mass_table_words( m, true ) );
+        arrays.place( m->mass_tables.lat32, mass_table_words( m, false ) );
+        arrays.place( m->mass_tables.rad32, mass_table_words( m, true ) );
+    }
     arrays.place( m->d_red_partials, size_t( kRedMaxBlocks ) * 8 );
     arrays.place( m->d_red_result, size_t( 16 ) );
     arrays.place( m->d_red_counter, size_t( 1 ) );
-    if ( ( rc = arrays.allocate( &m->d_block ) ) || ( rc = fill_tables( m ) ) )
+    if ( ( rc = arrays.allocate( &m->d_block ) ) || ( whole && ( rc = fill_tables( m ) ) ) )
     {
         tn_mesh_destroy( m );
         return rc;

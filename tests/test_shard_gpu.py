@@ -52,6 +52,19 @@ def _inputs(om):
     return k, src
 
 
+def test_shard_holds_no_tables_of_whole_shell_operators():
+    """device memory of one diamond at level 8: an ownership byte per node, and per column the points in both precisions,
+    ownership and group, with room for the allocator's 2 MiB pages; the whole-shell operators' tables would be 22 MB"""
+    from terraneo_b200.distributed import ShellShard
+    warm = ShellShard(2, 10, 0)
+    before = torch.cuda.mem_get_info()[0]
+    shard = ShellShard(8, 10, 3)
+    held = before - torch.cuda.mem_get_info()[0]
+    columns = shard.n1 ** 2
+    assert held <= columns * (shard.n1 + 24 + 12 + 1 + 4) + (6 << 20), held
+    del warm, shard
+
+
 @pytest.mark.parametrize("P", [1, 2, 3, 4, 8, 10])
 def test_shard_geometry_masks_and_ownership(P):
     from terraneo_b200.distributed import ShellShard
