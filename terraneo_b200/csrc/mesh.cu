@@ -203,6 +203,7 @@ WorkBlock::~WorkBlock()
 {
     if ( !p_ )
         return;
+    if ( n_ <= kKeptWork )
     {
         std::lock_guard< std::mutex > lock( m_->work_mutex );
         if ( n_ > m_->n_work )
