@@ -1,6 +1,9 @@
 """The kernels that run one thread per cell with the upper nodes handed to the lane above (cell.cuh), against the oracle
 at the levels where that can go wrong: partial warps and several columns per warp (1-3), one column per warp (5), a
-column over two warps (6); and the two-kernel CG (lateral_cg.cuh) against the oracle's iterates."""
+column over two warps (6); and the two-kernel CG (lateral_cg.cuh) against the oracle's iterates, with part of a tile per
+diamond (1-3), two tiles (4) and eight tiles and several runs of levels (5)."""
+import functools
+
 import numpy as np
 import pytest
 import torch
@@ -23,19 +26,25 @@ def _run(shell, op, pm, u, dtype, out_mesh=None, ncomp=None):
     return dst.numpy().reshape((3,) + dst.mesh.shape if dst.ncomp == 3 else dst.mesh.shape).astype(np.float64)
 
 
-@pytest.fixture(scope="module", params=LEVELS)
-def case(request):
+@functools.lru_cache(maxsize=None)
+def _case(L):
     from terraneo_b200 import shell
-    L = request.param
     om = Mesh(L)
-    return L, om, shell.ShellMesh(L), viscosity_field(om, seed=L), random_vector(om, seed=L)
+    return om, shell.ShellMesh(L), viscosity_field(om, seed=L), random_vector(om, seed=L)
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _release():
+    yield
+    _case.cache_clear()
 
 
 @pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
 @pytest.mark.parametrize("treat", [True, False])
-def test_divkgrad(case, treat, dtype):
+@pytest.mark.parametrize("L", LEVELS)
+def test_divkgrad(L, treat, dtype):
     from terraneo_b200 import shell
-    L, om, pm, k, u = case
+    om, pm, k, u = _case(L)
     kv = shell.VectorQ1Scalar(pm, dtype)
     kv.set_numpy(k)
     for single in (False, True) if L < 6 else (False,):
@@ -44,23 +53,24 @@ def test_divkgrad(case, treat, dtype):
 
 
 @pytest.mark.parametrize("treat", [True, False])
-def test_epsdivdiv3x2(case, treat):
+@pytest.mark.parametrize("L", LEVELS)
+def test_epsdivdiv3x2(L, treat):
     from terraneo_b200 import shell
-    L, om, pm, k, u = case
+    om, pm, k, u = _case(L)
     kv = shell.VectorQ1Scalar(pm)
     kv.set_numpy(k)
     assert rel(_run(shell, shell.EpsilonDivDiv(pm, kv, treat), pm, u, torch.float64),
                om.epsdivdiv3x2(k, u, treat)) <= 1e-12
 
 
-@pytest.mark.parametrize("kappa,treat,lumped", [(1e-3, True, False), (1e-6, False, False), (0.5, True, True),
-                                                (0.0, True, False)])
-def test_supg(case, kappa, treat, lumped):
+@pytest.mark.parametrize("L,kappa,treat,lumped",
+                         [(L, *p) for L in LEVELS[:-1] for p in ((1e-3, True, False), (1e-6, False, False),
+                                                                 (0.5, True, True), (0.0, True, False))]
+                         + [(6, 1e-3, True, False)])
+def test_supg(L, kappa, treat, lumped):
     """Peclet numbers from 1e-3 (the small-argument branch of tau) to 1e7; some nodes at rest"""
     from terraneo_b200 import shell
-    L, om, pm, k, u = case
-    if L == 6 and kappa != 1e-3:
-        return
+    om, pm, k, u = _case(L)
     vel = np.where(np.abs(u[:1]) > 1.5, 0.0, u)
     vv = shell.VectorQ1Vec(pm)
     vv.set_numpy(vel)
@@ -69,11 +79,10 @@ def test_supg(case, kappa, treat, lumped):
 
 
 @pytest.mark.parametrize("bc", [(1, 2), (2, 0)])
-def test_stokes_blocks(case, bc):
+@pytest.mark.parametrize("L", LEVELS[1:])  # the pressure mesh is one level coarser
+def test_stokes_blocks(L, bc):
     from terraneo_b200 import shell
-    L, om, pm, k, u = case
-    if L < 2:
-        return
+    om, pm, k, u = _case(L)
     oc, pc = Mesh(L - 1), shell.ShellMesh(L - 1)
     assert rel(_run(shell, shell.Divergence(pm, pc, *bc), pm, u, torch.float64, pc, 1),
                om.divergence(oc, u, *bc)) <= 1e-12
@@ -84,15 +93,16 @@ def test_stokes_blocks(case, bc):
     assert rel(vu.numpy(), om.gradient(oc, p, *bc)) <= 1e-12
 
 
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
 @pytest.mark.parametrize("bc", [(0, 0), (1, 2), (2, 0)])
-def test_viscosity_gradient(case, bc):
+@pytest.mark.parametrize("L", LEVELS)
+def test_viscosity_gradient(L, bc, dtype):
     """linear in k: d(lambda^T A(k) u)/dk times a perturbation of k, summed over the owned nodes, is lambda^T A(dk) u"""
     from terraneo_b200 import shell
-    L, om, pm, k, u = case
-    if L > 5:
-        return
-    lam, dk = random_vector(om, seed=L + 1), random_vector(om, seed=L + 2, ncomp=1)
-    vu, vl, g = shell.VectorQ1Vec(pm), shell.VectorQ1Vec(pm), shell.VectorQ1Scalar(pm)
+    om, pm, _, _ = _case(L)
+    u, lam = (random_vector(om, seed=L + i).astype(np.float32).astype(np.float64) for i in (0, 1))
+    dk = random_vector(om, seed=L + 2, ncomp=1)
+    vu, vl, g = shell.VectorQ1Vec(pm, dtype), shell.VectorQ1Vec(pm, dtype), shell.VectorQ1Scalar(pm, dtype)
     vu.set_numpy(u)
     vl.set_numpy(lam)
     shell.epsdivdiv_kgrad(pm, *bc, vu, vl, g)
@@ -100,16 +110,14 @@ def test_viscosity_gradient(case, bc):
     terms = om.kerngen(dk, u, *bc) * lam
     want = float((terms * own).sum())
     # a sum of N terms of both signs: bounded by their absolute sum
-    assert abs(float((g.numpy()[0] * dk * own).sum()) - want) <= 1e-12 * float(np.abs(terms * own).sum())
+    assert abs(float((g.numpy()[0] * dk * own).sum()) - want) <= TOL[dtype] * float(np.abs(terms * own).sum())
 
 
-@pytest.mark.parametrize("its", [1, 2, 9, 17])
-def test_cg_iterates(case, its):
-    """the iterate after 1, 2 (each direction field), 9 and 17 (the stopping flag is looked at every 8) steps"""
+@pytest.mark.parametrize("L,its", [(L, i) for L in (1, 2, 3) for i in (1, 2, 9, 17)] + [(4, 2), (4, 9), (5, 2), (5, 9)])
+def test_cg_iterates(L, its):
+    """the iterate after 1, 2 (each direction field), 9 and 17 (the stopping flag is looked at by then) steps"""
     from terraneo_b200 import shell
-    L, om, pm, k, u = case
-    if L > 3:
-        return
+    om, pm, k, u = _case(L)
     b = om.kmass(np.ones(om.shape), u[0], 0)
     b[..., 0] = b[..., -1] = 0.0
     vb, vx = shell.VectorQ1Scalar(pm), shell.VectorQ1Scalar(pm)

@@ -1,6 +1,7 @@
 """The separated form of the constant-coefficient operators (Laplace, VectorLaplace, mass matrix) against the oracle,
-copy by copy: every level whose block of 254 nodes ends inside a column or spans several, inputs whose duplicated
-nodes hold different values, and each apply / communication mode."""
+copy by copy: part of a tile of 8 x 16 columns per diamond (levels 1-3), two tiles (4) and eight (5), in one run of
+levels (1, 2), with a shorter last run (3, 4) and in three equal ones (5), inputs whose duplicated nodes hold different
+values, and each apply / communication mode; their CG (lateral_cg.cuh), tables and memory."""
 import numpy as np
 import pytest
 import torch
