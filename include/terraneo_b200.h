@@ -386,8 +386,9 @@ typedef struct
 
 /* entries of one FV field: 10 (N+2)^3 */
 TN_API int tn_fv_field_size( const tn_mesh* mesh, size_t* entries );
-/* doubles of the tn_fct_step_f64 workspace: 9 FV fields (T^L, 6 antidiffusive
- * fluxes per cell, R+, R-) */
+/* doubles of the tn_fct_step_f64 workspace: 9 FV fields (T^L, the antidiffusive
+ * fluxes, R+, R-; the fluxes take three of the six fields kept for them, one
+ * value per face) */
 TN_API int tn_fct_workspace_size( const tn_mesh* mesh, size_t* entries );
 /* update_fv_ghost_layers (communication/shell/fv_communication.hpp): lateral
  * ghost cells := the real cells across each diamond face */

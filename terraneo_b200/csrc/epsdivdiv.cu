@@ -22,8 +22,7 @@
 // boundary treatment decouples enter with zero; their diagonal comes from
 // further blocks of the launch (one thread per lateral cell, wedge and side).
 // Level-6 apply with its halo: FP64 1,067 -> 246 us, FP32 577 -> 153 us, bound by
-// instruction issue; four resident blocks per SM (128 registers, some spilled)
-// beat three (168) by 5 % and two by 20 %.
+// instruction issue.
 #include "cell.cuh"
 #include "common.cuh"
 #include "wedge.cuh"
@@ -198,8 +197,8 @@ __device__ __forceinline__ void epsdivdiv_diagonal( const E32Params< T >& P, int
             atomicAdd( P.dst.p[c] + id[m] + top, o[m][c] * P.src.p[c][id[m] + top] );
 }
 
-// Blocks per SM, level 6: FP64 at 3 / 4 / 5 blocks 248 / 252 / 319 us (spills from 4 on), FP32 at 4 / 5 / 6 165 / 155 /
-// 153 us.
+// Blocks per SM, level 6: FP64 at 3 / 4 / 5 blocks 248 / 252 / 319 us (36 bytes spilled at 3, more above), FP32 at 4 / 5 /
+// 6 165 / 155 / 153 us (24 bytes at 6).
 template < typename T >
 __global__ void __launch_bounds__( 128, sizeof( T ) == 8 ? 3 : 6 ) epsdivdiv3x2_kernel( E32Params< T > P )
 {

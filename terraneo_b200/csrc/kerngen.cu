@@ -723,8 +723,10 @@ __global__ void __launch_bounds__( 128 ) kerngen_cell_kernel( CellParams< T > P 
 // (it leaves these cells out).  A block takes kBcX x kBcY cells of one layer
 // (y fastest) and adds its cells' contributions to a node in shared memory
 // first, one atomic per node and component for up to four cells: the nodes of a
-// layer lie a column apart, so each of these atomics is its own sector and their
-// rate in L2 is what bounds the kernel (24 per cell without that, 7.2 with it).
+// layer lie a column apart, so each of these atomics is its own sector (24 per cell
+// without that, 7.2 with it; L2 at 42 -> 24 % FP64, 45 -> 29 % FP32).  What is left
+// is the latency of the loads, as scattered and four times repeated as before (29
+// sectors per request, long scoreboard first among the stalls).
 // Kernel time: FP64 Dirichlet level 6 24.2 -> 20.8 us, FP32 free-slip level 5 9.0 ->
 // 6.7 us and level 7 85 -> 76 us.
 constexpr int kBcX = 8, kBcY = 16;

@@ -144,7 +144,7 @@ __device__ __forceinline__ void divkgrad_diagonal( const DivKGradParams< T >& P,
 // boundary treatment the CMB nodes of layer 0 (otherwise the SURFACE nodes of
 // layer N - 1) enter with zero and keep their diagonal, which further blocks of the
 // launch add (one thread per lateral cell, wedge and side).  Blocks per SM, FP64: at 4 / 5 / 6 95 / 91 / 97 us at
-// level 6, 689 / 642 / 670 us at level 7.
+// level 6, 689 / 642 / 670 us at level 7; FP32 takes 70 registers whatever the bound (seven blocks).
 template < typename T, bool SINGLE >
 __global__ void __launch_bounds__( 128, 5 ) divkgrad_kernel( DivKGradParams< T > P )
 {

@@ -14,7 +14,7 @@
 // level 6, no longer at level 5.
 // Per iteration: the Laplacian at level 5 38 us of kernels (apply, halo, product,
 // update, direction; 61 us with the gaps) -> 24 us, the mass matrix at level 6 350 us
-// with two host reads -> 80 us.
+// with two host reads -> 83 us.
 #pragma once
 
 #include "lateral.cuh"
