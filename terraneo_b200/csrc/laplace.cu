@@ -339,7 +339,7 @@ int constant_gradient_apply( const tn_mesh* m, int nc, const T* const* src, T* c
         P.src.p[c] = src[c];
         P.dst.p[c] = dst[c];
     }
-    if ( !lateral_tables< LaplaceOp< T > >( m, &tn_mesh::laplace_tables, P, st ) )
+    if ( !lateral_tables< LaplaceOp< T > >( m, &tn_mesh::laplace_tables, P ) )
     {
         set_error( std::string( what ) + ": allocating the lateral stencils failed" );
         return TN_ERR_NOMEM;
@@ -376,7 +376,7 @@ int laplace_cg( const tn_mesh* m, const double* b, double* x, int max_iterations
                 double* relres, cudaStream_t st )
 {
     LateralParams< double > P{};
-    if ( !lateral_tables< LaplaceOp< double > >( m, &tn_mesh::laplace_tables, P, st ) )
+    if ( !lateral_tables< LaplaceOp< double > >( m, &tn_mesh::laplace_tables, P ) )
     {
         set_error( "laplace_cg: allocating the lateral stencils failed" );
         return TN_ERR_NOMEM;

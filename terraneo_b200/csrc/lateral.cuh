@@ -595,35 +595,46 @@ bool lateral_fill( const tn_mesh* m, const LateralTables& t, cudaStream_t st )
     return cudaGetLastError() == cudaSuccess;
 }
 
-// An operator's tables in the precision of T, built on the mesh's first use of them and complete for every stream
-// when this returns; false when that fails.
+// An operator's tables in the precision of T, built on the mesh's first use of them and complete for every stream when
+// this returns; false when that fails.  The first use may lie in a stream capture (that of another precision or of an
+// operator that shares no table may have come before it): the fill runs on a stream of its own, and allocating is allowed
+// to this thread meanwhile.
 template < typename OP, typename T >
-bool lateral_tables( const tn_mesh* m, tn_lateral_tables tn_mesh::*which, LateralParams< T >& P, cudaStream_t st )
+bool lateral_tables( const tn_mesh* m, tn_lateral_tables tn_mesh::*which, LateralParams< T >& P )
 {
+    struct AllowAllocation
+    {
+        cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+        AllowAllocation() { cudaThreadExchangeStreamCaptureMode( &mode ); }
+        ~AllowAllocation() { cudaThreadExchangeStreamCaptureMode( &mode ); }
+    };
     tn_mesh*                      mm = const_cast< tn_mesh* >( m );
     std::lock_guard< std::mutex > lock( mm->geom_mutex );
     tn_lateral_tables&            t    = mm->*which;
     T *&                          dlat = lateral_slot< T >( t.lat, t.lat32 ), *&drad = lateral_slot< T >( t.rad, t.rad32 );
     if ( !dlat )
     {
-        T *l = nullptr, *r = nullptr;
-        if ( cudaMalloc( &l, lateral_table_words< OP >( m, false ) * sizeof( T ) ) != cudaSuccess ||
-             cudaMalloc( &r, lateral_table_words< OP >( m, true ) * sizeof( T ) ) != cudaSuccess )
+        const AllowAllocation allow;
+        const size_t          words = lateral_table_words< OP >( m, false );
+        T*                    l     = nullptr; // the stencils, then the radial factors
+        cudaStream_t          st    = nullptr;
+        LateralTables         out{};
+        bool ok = cudaMalloc( &l, ( words + lateral_table_words< OP >( m, true ) ) * sizeof( T ) ) == cudaSuccess &&
+                  cudaStreamCreateWithFlags( &st, cudaStreamNonBlocking ) == cudaSuccess;
+        if ( ok )
+        {
+            lateral_slot< T >( out.lat, out.lat32 ) = l, lateral_slot< T >( out.rad, out.rad32 ) = l + words;
+            ok = lateral_fill< OP >( m, out, st ) && cudaStreamSynchronize( st ) == cudaSuccess;
+        }
+        if ( st )
+            cudaStreamDestroy( st );
+        if ( !ok )
         {
             (void) cudaGetLastError();
             cudaFree( l );
             return false;
         }
-        LateralTables out{};
-        lateral_slot< T >( out.lat, out.lat32 ) = l, lateral_slot< T >( out.rad, out.rad32 ) = r;
-        if ( !lateral_fill< OP >( m, out, st ) || cudaStreamSynchronize( st ) != cudaSuccess )
-        {
-            (void) cudaGetLastError();
-            cudaFree( l );
-            cudaFree( r );
-            return false;
-        }
-        dlat = l, drad = r;
+        dlat = l, drad = l + words;
     }
     P.lat = dlat, P.rad = drad;
     return true;

@@ -157,7 +157,7 @@ int kmass_apply( const tn_mesh* m, const T* k, int mode, int apply_mode, int com
     {
         LateralParams< T > P{};
         P.src.p[0] = src, P.dst.p[0] = dst, P.mode_first = P.mode_inner = P.mode_last = mode == 1 ? kDiag : kNeu;
-        if ( !lateral_tables< MassOp< T > >( m, &tn_mesh::mass_tables, P, st ) )
+        if ( !lateral_tables< MassOp< T > >( m, &tn_mesh::mass_tables, P ) )
         {
             set_error( "kmass: allocating the lateral stencil failed" );
             return TN_ERR_NOMEM;
@@ -194,7 +194,7 @@ int mass_cg( const tn_mesh* m, const double* b, double* x, double* fields, int m
              int* iterations, cudaStream_t st )
 {
     LateralParams< double > P{};
-    if ( !lateral_tables< MassOp< double > >( m, &tn_mesh::mass_tables, P, st ) )
+    if ( !lateral_tables< MassOp< double > >( m, &tn_mesh::mass_tables, P ) )
     {
         set_error( "mass_cg: allocating the lateral stencil failed" );
         return TN_ERR_NOMEM;

@@ -547,9 +547,8 @@ extern "C" int tn_mesh_destroy( tn_mesh* m )
         return TN_OK;
     cudaFree( m->d_block );
     cudaFree( m->d_fv_orient );
-    for ( void* p : { static_cast< void* >( m->laplace_tables.lat ), static_cast< void* >( m->laplace_tables.rad ),
-                      static_cast< void* >( m->laplace_tables.lat32 ), static_cast< void* >( m->laplace_tables.rad32 ) } )
-        cudaFree( p );
+    cudaFree( m->laplace_tables.lat ); // with its radial factors
+    cudaFree( m->laplace_tables.lat32 );
     cudaFree( m->d_work );
     if ( m->h_red_result )
         cudaFreeHost( m->h_red_result );

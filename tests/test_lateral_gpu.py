@@ -52,18 +52,25 @@ def test_every_copy_and_mode(op, bc, L, dtype, tol):
     assert rel(_apply(*args, C.APPLY_ADD, C.COMM_ADDITIVE), halo(own + old)) <= tol
 
 
-def test_first_mass_apply_in_a_capture():
-    """nothing is allocated or waited for on a mesh's first mass apply, so it may be part of a graph"""
+@pytest.mark.parametrize("op", ["mass", "laplace", "vector_laplace"])
+@pytest.mark.parametrize("dtype", [torch.float64, torch.float32])
+def test_first_apply_in_a_capture(op, dtype):
+    """a mesh's first use of an operator's tables in a precision may be part of a graph, whatever was used before it"""
     from terraneo_b200 import shell
+    cls = shell.VectorQ1Vec if op == "vector_laplace" else shell.VectorQ1Scalar
+    make = {"mass": lambda m: shell.KMass(m), "laplace": lambda m: shell.Laplace(m, True),
+            "vector_laplace": lambda m: shell.VectorLaplace(m, 1, 1)}[op]
     pm, warm = shell.ShellMesh(3), shell.ShellMesh(2)
-    shell.apply(shell.KMass(warm), *(shell.VectorQ1Scalar(warm) for _ in range(2)))  # the module is loaded outside
-    src, dst, ref = (shell.VectorQ1Scalar(pm) for _ in range(3))
+    shell.apply(make(warm), *(cls(warm, dtype) for _ in range(2)))  # the module is loaded outside
+    other = torch.float32 if dtype == torch.float64 else torch.float64
+    shell.apply(make(pm), *(cls(pm, other) for _ in range(2)))
+    src, dst, ref = (cls(pm, dtype) for _ in range(3))
     src.data.uniform_()
     graph = torch.cuda.CUDAGraph()
     with torch.cuda.graph(graph):
-        shell.apply(shell.KMass(pm), src, dst)
+        shell.apply(make(pm), src, dst)
     graph.replay()
-    shell.apply(shell.KMass(pm), src, ref)
+    shell.apply(make(pm), src, ref)
     torch.cuda.synchronize()
     assert torch.equal(dst.data, ref.data)
 
