@@ -36,12 +36,15 @@ __global__ void __launch_bounds__( kLateralThreads, 4 ) lateral_cg_kernel( Later
     block_sum_finish< 1 >( &dot, cg.partials, cg.counter, cg.state + 1 ); // pap
 }
 
+// steps after which the residual history of tn_pcg_* (which nothing reads here) is written over from its start
+constexpr int kLateralHistory = 4096;
+
 // doubles of the work array of lateral_cg besides its four fields r, p, p', ap
 template < typename OP >
 size_t lateral_cg_scratch( const tn_mesh* m, int max_iterations )
 {
     LateralParams< double > P{};
-    return 2 * size_t( lateral_shape( m, true, P ) ) + 2 + 8 + size_t( std::max( max_iterations, 0 ) ) + 1;
+    return 2 * size_t( lateral_shape( m, true, P ) ) + 2 + 8 + size_t( std::clamp( max_iterations, 0, kLateralHistory ) ) + 1;
 }
 
 // Solves A x = b from x's values; P: the operator's tables and layer modes.  fields: r, p, p', ap (stored nodes each);
@@ -89,7 +92,8 @@ int lateral_cg( const tn_mesh* m, LateralParams< double > P, const double* b, do
     TN_CUDA_TRY( cudaEventCreateWithFlags( &ev, cudaEventDisableTiming ) );
     double* const flag    = m->h_red_result + 15;
     bool          pending = false;
-    for ( int it = 0; it < max_iterations && rc == TN_OK; ++it )
+    int           it      = 0;
+    for ( ; it < max_iterations && rc == TN_OK; ++it )
     {
         if ( it == 2 || ( it > 0 && it % kEvery == 0 ) )
         {
@@ -107,7 +111,7 @@ int lateral_cg( const tn_mesh* m, LateralParams< double > P, const double* b, do
             rc = TN_ERR_CUDA;
             break;
         }
-        rc = tn_pcg_update_f64( 1, mm, xx, rr, pp, aa, cg.state, 0, rtol, atol, st );
+        rc = tn_pcg_update_f64( 1, mm, xx, rr, pp, aa, cg.state, it % kLateralHistory + 1, rtol, atol, st );
     }
     cudaEventDestroy( ev );
     if ( rc )
@@ -115,8 +119,9 @@ int lateral_cg( const tn_mesh* m, LateralParams< double > P, const double* b, do
     double out[2];
     TN_CUDA_TRY( cudaMemcpyAsync( out, cg.state + 5, sizeof( out ), cudaMemcpyDeviceToHost, st ) );
     TN_CUDA_TRY( cudaStreamSynchronize( st ) );
+    // out[0] counts modulo kLateralHistory, and at most 16 of the `it` steps issued come after the last one taken
     if ( iterations )
-        *iterations = int( out[0] );
+        *iterations = out[0] == 0.0 ? 0 : it - ( it - int( out[0] ) ) % kLateralHistory;
     if ( relres )
         *relres = out[1];
     return TN_OK;

@@ -248,3 +248,37 @@ def test_solver_memory_is_given_back(L, kept):
     for _ in range(3):
         shell.laplace_pcg(pm, b, x, 2)
     assert before - torch.cuda.mem_get_info()[0] <= kept + (4 << 20)
+
+
+@pytest.mark.parametrize("solve", ["laplace", "projection"])
+def test_cg_with_any_iteration_limit(solve):
+    """the limit sizes no memory (17 GB at the largest when every step had an entry): such a call takes no longer than one
+    with a small limit; and steps are counted beyond the kept history of 4,096"""
+    import time
+    from terraneo_b200 import shell
+    pm = shell.ShellMesh(2)
+    b, x = shell.VectorQ1Scalar(pm), shell.VectorQ1Scalar(pm)
+    x.data.normal_()
+    shell.apply(shell.KMass(pm), x, b)  # equal copies of every node: the system has a solution
+    b.data[..., 0] = b.data[..., -1] = 0.0
+    fv = torch.randn((10,) + (pm.n1 + 1,) * 3, dtype=torch.float64, device="cuda")
+
+    def run(its, rtol, atol):
+        best, n = 1e9, 0
+        for _ in range(4):
+            x.data.zero_()
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            if solve == "laplace":
+                n, _ = shell.laplace_pcg(pm, b, x, its, rtol, atol)
+            else:
+                n = shell.l2_project_fv_to_fe(pm, fv, x, False, its, rtol, atol)
+            best = min(best, time.perf_counter() - t)
+        return n, best
+
+    n, small = run(1000, 1e-10, 1e-30)
+    assert 0 < n < 1000
+    free = torch.cuda.mem_get_info()[0]
+    m, large = run(2**31 - 1, 1e-10, 1e-30)
+    assert m == n and large <= small + 1e-3 and free - torch.cuda.mem_get_info()[0] <= 4 << 20, (n, m, small, large)
+    assert run(4096, -1.0, 0.0)[0] == 4096 and run(4100, -1.0, 0.0)[0] == 4100  # never met
